@@ -58,8 +58,11 @@ typedef struct radm2_opts {
     int precision;      /* RADM2_PREC_* (default FP64) */
     int refine_sweeps;  /* FP32LU: FP64 refinement sweeps per stage solve, 0..2 (default 1) */
     int schedule;       /* RADM2_SCHED_* (default STATIC) */
-    int block_threads;  /* threads per block: 0 = default (128; 256 for RADM2_SCHED_COOP);
-                           32, 64, 128 or 256 (the built variants) */
+    int block_threads;  /* threads per block: 32, 64, 128 or 256 (the built variants), or 0 = the
+                           library's launch shape: for FP64 with global placement and no other
+                           shape option the wide tensor-memory kernel (either schedule; its own
+                           128-thread CTAs, cells from a queue), else 128 (256 for
+                           RADM2_SCHED_COOP) */
     int blocks_per_sm;  /* persistent grid blocks per SM: 0 = default */
     int float_coeffs;   /* 1 (default): M/E rounded through float as mgpu.cu:3300-3304 */
     int placement;      /* working-set placement: RADM2_PLACE_* (default GLOBAL) */

@@ -18,6 +18,7 @@ struct radm2_ctx {
     double *var = nullptr, *fix = nullptr, *temp = nullptr, *rcn = nullptr, *jv = nullptr, *rconst = nullptr;
     bool have_rcn = false;
     bool rconst_valid = false;
+    bool rconst_formula = true;  // the rate constants (once valid) are the formulas' own, not radm2_set_rconst's
     double *h0 = nullptr;
     int *order = nullptr;
     int *status = nullptr, *nacc = nullptr, *nrej = nullptr;

@@ -7,6 +7,19 @@
 
 #include "gen/radm2_gen.h"
 
+// c += a b and c -= a b of the generated sums: one rounding, or two in the files that are built
+// without multiply-add contraction (--fmad=false goes with -DRADM2_FUSED=0).
+#ifndef RADM2_FUSED
+#define RADM2_FUSED 1
+#endif
+#if RADM2_FUSED
+#define FMAC(c, a, b) c = fma(a, b, c)
+#define FNMA(c, a, b) c = fma(-(a), b, c)
+#else
+#define FMAC(c, a, b) c = c + (a) * (b)
+#define FNMA(c, a, b) c = c - (a) * (b)
+#endif
+
 namespace radm2 {
 
 constexpr int NVAR = RADM2_NVAR;

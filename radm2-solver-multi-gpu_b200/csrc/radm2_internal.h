@@ -67,6 +67,12 @@ cudaError_t launch_solver_coop_g4(const SolveArgs &a, int grid, cudaStream_t st)
 cudaError_t launch_solver_coop_g8(const SolveArgs &a, int grid, cudaStream_t st);
 cudaError_t launch_solver_coopx_g8(const SolveArgs &a, int grid, cudaStream_t st);
 
+// The wide tensor-memory solver (radm2_wide.cuh): FP64, one 128-thread CTA per SM, cells from
+// the work queue; needs rate constants that come from the mechanism's formulas (repeated ones
+// are stored once).  The "x" kernel keeps the reference's arithmetic.
+cudaError_t launch_solver_wide(const SolveArgs &a, int grid, cudaStream_t st);
+cudaError_t launch_solver_widex(const SolveArgs &a, int grid, cudaStream_t st);
+
 // Two cells per thread (radm2_solver_cpt2.cuh): FP64, global placement, bs 64 or 128,
 // sched 0 static / 1 persistent.
 cudaError_t launch_solver_cpt2(const SolveArgs &a, int bs, int sched, int grid, cudaStream_t st);
@@ -105,6 +111,8 @@ cudaError_t solver_info_fp64x_static(int key, SolverInfo *out);
 cudaError_t solver_info_fp64x_persistent(int key, SolverInfo *out);
 cudaError_t solver_info_cpt2(int bs, int sched, SolverInfo *out);
 int solver_layout_check_cpt2();
+cudaError_t solver_info_wide(SolverInfo *out);
+cudaError_t solver_info_widex(SolverInfo *out);
 cudaError_t solver_info_coop_g4(SolverInfo *out);
 cudaError_t solver_info_coop_g8(SolverInfo *out);
 cudaError_t solver_info_coopx_g8(SolverInfo *out);

@@ -183,6 +183,24 @@ def check_jacvec(m, chains, uses):
 
 # ----------------------------------------------------------------------------- CUDA fragments
 
+def fused_add(r, var, op, term, product):
+    """The statement var op= term, with the term's last product fused where the build contracts
+    multiply-adds (FMAC / FNMA in radm2_device.cuh).  product: the expression of the rate or partial
+    that the term scales.  Written out because the compiler may fuse either product of a sum's
+    first addition, by their numbers of uses: kernels that share these sums must round alike."""
+    if term[0] == "neg":
+        term, op = term[1], "-" if op == "+" else "+"
+    if term[0] == "ref":
+        if product[0] != "bin":
+            return "%s = (%s %s %s);" % (var, var, op, r(term))
+        a, b = product[2], product[3]
+    else:
+        a, b = term[2], term[3]
+        if a[0] == "neg":
+            a, op = a[1], "-" if op == "+" else "+"
+    return "%s(%s, %s, %s);" % ("FMAC" if op == "+" else "FNMA", var, r(a), r(b))
+
+
 def kernel_ref(arr, i):
     return {"RCT": "RC(%d)", "V": "V(%d)", "F": "FIX(%d)", "A": "a%d", "B": "b%d",
             "jv": "JV(%d)", "XIN": "XIN(%d)", "DA": "da%d"}[arr] % i
@@ -231,8 +249,8 @@ def emit_cuda(m, out_dir):
     # its reactions in increasing order, so accumulating in reaction order applies the
     # same binary operations to each accumulator in the same order as the reference's
     # left-to-right sum (bit-identical), while only 59 accumulators stay live.
-    body = [BANNER, "/* ODE right-hand side, mgpu.cu:1103-1385, reaction-major.  Inputs: RC(r), V(i), FIX(k).\n"
-            " * Output VDOT_OUT(i, value) after all reactions. */\n"]
+    body = [BANNER, "/* ODE right-hand side, mgpu.cu:1103-1385, reaction-major.  Inputs: RC(r), V(i), FIX(k);\n"
+            " * FMAC, FNMA.  Output VDOT_OUT(i, value) after all reactions. */\n"]
     f = 0
     chains = []
     for i, t in enumerate(m["vdot"]):
@@ -270,7 +288,7 @@ def emit_cuda(m, out_dir):
             if pos == 0:
                 body.append("  vd%d = %s;\n" % (i, r(term)))
             else:
-                body.append("  vd%d = (vd%d %s %s);\n" % (i, i, op, r(term)))
+                body.append("  %s\n" % fused_add(r, "vd%d" % i, op, term, t))
         body.append("}\n")
     for i in range(len(chains)):
         body.append("VDOT_OUT(%d, vd%d);\n" % (i, i))
@@ -285,7 +303,7 @@ def emit_cuda(m, out_dir):
     # slots use JAC_OUT_ZERO(s, is_diag).
     dset = set(diag)
     body = [BANNER, "/* Sparse Jacobian in LU slot order, mgpu.cu:1685-2652, partial-major.\n"
-            " * Inputs: RC(r), V(i), FIX(k). */\n"]
+            " * Inputs: RC(r), V(i), FIX(k); FMAC, FNMA. */\n"]
     f = 0
     juses = {}
     last_b = {}
@@ -325,13 +343,14 @@ def emit_cuda(m, out_dir):
             if pos == 0:
                 expr = r(term)
             else:
-                expr = "(js%d %s %s)" % (sl, op, r(term))
+                expr = "js%d" % sl
+                body.append("  %s\n" % fused_add(r, expr, op, term, bt))
+                if not is_last:
+                    continue
             if is_last:
                 body.append("  %s(%d, %s);\n" % ("JAC_OUT_DIAG" if sl in dset else "JAC_OUT", sl, expr))
-            elif pos == 0:
-                body.append("  double js%d = %s;\n" % (sl, expr))
             else:
-                body.append("  js%d = %s;\n" % (sl, expr))
+                body.append("  double js%d = %s;\n" % (sl, expr))
         body.append("}\n")
     flops["jac"] = f
     # declarations of the open accumulators must precede their first use: hoist them.
