@@ -7,12 +7,13 @@
 // reference's divisions, built without contraction.
 //
 // What bounds it and why it is built this way (B200, 262,144 mixed cells, one 600 s step):
-//   Instruction fetch.  A step attempt is straight-line code, so an SM streams all of it once
-//   per attempt.  Measured on straight-line code beyond 128 KB: 6.1 cycles per instruction for
-//   a warp, the same for 4 or 8 warps that run the same lines together, 12.5 for 4 warps on
-//   lines of their own.  So the block starts every attempt together (a block-wide vote ends
-//   the loop; barriers inside the phases measured 3-20% slower), the RHS and the solve exist
-//   once and run in a loop over the stages, and the error norm is a small loop.
+//   Instruction fetch.  A step attempt is straight-line code (200 KB), so an SM streams all of
+//   it once per attempt.  Measured on straight-line code beyond 128 KB: 6.1 cycles per
+//   instruction for one warp, the same for 4 or 8 warps that run the same lines together, 12.5
+//   for 4 warps on lines of their own.  So fewer instructions are faster whatever they do: the
+//   RHS and the solve exist once and run in a loop over the stages, and the error norm is a
+//   small loop.  Keeping the warps together costs more than it gives: a block-wide vote per
+//   attempt takes 86 ms instead of 83, barriers inside the phases 90-110 ms.
 //   Memory latency.  One warp per scheduler hides nothing, so the generated phases issue
 //   their global loads about 100 operations ahead and each tensor-memory group while the
 //   previous one is used.
@@ -173,8 +174,7 @@ __global__ void __launch_bounds__(WIDE_BS, 1) k_rosenbrock_wide(const SolveArgs 
             H = mind(H, absd(P.Tend - T));
             outer = false;
         }
-        __syncwarp();
-        if (!__syncthreads_or(have)) break;
+        if (!__any_sync(0xffffffffu, have)) break;
 
         // ---------------------------------------------------------------- one attempt
         // Every lane runs it (tensor-memory accesses are warp-collective); a lane without an
@@ -249,19 +249,16 @@ __global__ void __launch_bounds__(WIDE_BS, 1) k_rosenbrock_wide(const SolveArgs 
                 for (int i = 0; i < NVAR; i++) asm volatile("" : "+d"(x[i]));  // F is rounded before it is used
             }
             if (stage == 1) {
+                constexpr int A = 30;  // loads in flight
+                double k1[NVAR];
 #pragma unroll
-                for (int h = 0; h < NVAR; h += 30) {
-                    double k1[30];
-#pragma unroll
-                    for (int i = 0; i < 30; i++)
-                        if (h + i < NVAR) GLDI(k1[i], gp, RADM2_WIDE_GK1 + h + i);
-#pragma unroll
-                    for (int i = 0; i < 30; i++)
-                        if (h + i < NVAR) {
-                            const double f = x[h + i];
-                            x[h + i] = f + k1[i] * hc21;
-                            V(h + i) = f + k1[i] * hc31;
-                        }
+                for (int i = 0; i < NVAR + A; i++) {
+                    if (i < NVAR) GLDI(k1[i], gp, RADM2_WIDE_GK1 + i);
+                    if (i >= A) {
+                        const double f = x[i - A];
+                        x[i - A] = f + k1[i - A] * hc21;
+                        V(i - A) = f + k1[i - A] * hc31;
+                    }
                 }
             }
             if (stage == 2) {
@@ -285,64 +282,55 @@ __global__ void __launch_bounds__(WIDE_BS, 1) k_rosenbrock_wide(const SolveArgs 
         for (int i = 0; i < NVAR; i++) V(i) = x[i];  // K3
         double err = 0.0;
         {
-            constexpr int U = 4;
+            constexpr int U = 4, END = (NVAR + U - 1) / U * U;
+            static_assert(END - NVAR < U && RADM2_WIDE_GY + END <= WIDE_GLOBAL_WORDS, "the last step reads past the species");
             double k0[U], k1[U], y[U];
             const double *g = gp;
-            auto load = [&](int n) {
+            auto load = [&]() {
 #pragma unroll
-                for (int j = 0; j < U; j++)
-                    if (j < n) {
-                        GLDI(k0[j], g, RADM2_WIDE_GK1 + j);
-                        GLDI(k1[j], g, RADM2_WIDE_GK2 + j);
-                        GLDI(y[j], g, RADM2_WIDE_GY + j);
-                    }
-                g += n * WIDE_BS;
+                for (int j = 0; j < U; j++) {
+                    GLDI(k0[j], g, RADM2_WIDE_GK1 + j);
+                    GLDI(k1[j], g, RADM2_WIDE_GK2 + j);
+                    GLDI(y[j], g, RADM2_WIDE_GY + j);
+                }
+                g += U * WIDE_BS;
             };
-            auto step = [&](int i, int n, bool next) {
+            load();
+#pragma unroll 1
+            for (int i = 0; i < END; i += U) {
                 double num[U], den[U], q[U];
                 int top = 0, low = 0x7fffffff;
 #pragma unroll
-                for (int j = 0; j < U; j++)
-                    if (j < n) {
-                        const double k2 = V(i + j);
-                        const double ynew = P.M[0] * k0[j] + P.M[1] * k1[j] + P.M[2] * k2 + y[j];
-                        const double yerr = P.E[0] * k0[j] + P.E[1] * k1[j] + P.E[2] * k2;
-                        const double ymax = maxd(fabs(y[j]), fabs(ynew));
-                        const double scale = P.AbsTol[i + j] + P.RelTol[i + j] * ymax;
-                        num[j] = yerr * yerr;
-                        den[j] = scale * scale;
-                        V(i + j) = ynew;
-                    }
-                if (next) load(U);
+                for (int j = 0; j < U; j++) {
+                    const bool in = j < U - (END - NVAR) || i + j < NVAR;  // the last step is not full
+                    const double k2 = V(i + j);
+                    const double ynew = P.M[0] * k0[j] + P.M[1] * k1[j] + P.M[2] * k2 + y[j];
+                    const double yerr = P.E[0] * k0[j] + P.E[1] * k1[j] + P.E[2] * k2;
+                    const double ymax = maxd(fabs(y[j]), fabs(ynew));
+                    const double scale = P.AbsTol[i + j] + P.RelTol[i + j] * ymax;
+                    num[j] = in ? yerr * yerr : 0.0;
+                    den[j] = in ? scale * scale : 1.0;
+                    if (in) V(i + j) = ynew;
+                }
+                if (i + U < END) load();
 #if RADM2_WIDE_DIV
 #pragma unroll
-                for (int j = 0; j < U; j++)
-                    if (j < n) q[j] = num[j] / den[j];
+                for (int j = 0; j < U; j++) q[j] = num[j] / den[j];
 #else
 #pragma unroll
-                for (int j = 0; j < U; j++)
-                    if (j < n) {
-                        q[j] = div_newton(num[j], den[j]);
-                        top = max(top, max(__double2hiint(num[j]), __double2hiint(den[j])));
-                        low = min(low, __double2hiint(den[j]));
-                    }
+                for (int j = 0; j < U; j++) {
+                    q[j] = div_newton(num[j], den[j]);
+                    top = max(top, max(__double2hiint(num[j]), __double2hiint(den[j])));
+                    low = min(low, __double2hiint(den[j]));
+                }
                 if (top > DIV_NEWTON_TOP || low < DIV_NEWTON_LOW) {
 #pragma unroll
-                    for (int j = 0; j < U; j++)
-                        if (j < n) q[j] = div_exact(num[j], den[j]);
+                    for (int j = 0; j < U; j++) q[j] = div_exact(num[j], den[j]);
                 }
 #endif
 #pragma unroll
-                for (int j = 0; j < U; j++)
-                    if (j < n) err += q[j];
-            };
-            load(U);
-#pragma unroll 1
-            for (int i = 0; i < NVAR - U; i += U) step(i, U, i + 2 * U <= NVAR);
-            constexpr int R = NVAR % U;
-            static_assert(R > 0, "the last step takes the remaining species");
-            load(R);
-            step(NVAR - R, R, false);
+                for (int j = 0; j < U; j++) err += q[j];
+            }
         }
 
         // Step control (mgpu.cu:3240-3260).
@@ -372,12 +360,12 @@ __global__ void __launch_bounds__(WIDE_BS, 1) k_rosenbrock_wide(const SolveArgs 
             }
         }
         if (!take) {  // the state back in its place
-#pragma unroll 8
-            for (int i = 0; i < NVAR; i++) {
-                double y;
-                GLDI(y, gp, RADM2_WIDE_GY + i);
-                V(i) = y;
-            }
+#pragma unroll
+            for (int i = 0; i < NVAR; i++)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(sa + i * (WIDE_BS * 8)),
+                             "l"(gp + (RADM2_WIDE_GY + i) * WIDE_BS)
+                             : "memory");
+            asm volatile("cp.async.wait_all;" ::: "memory");
         }
     }
     // every warp is done with its tensor memory: warp 0 frees it

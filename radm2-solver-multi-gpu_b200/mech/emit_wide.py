@@ -13,9 +13,9 @@ The mechanism's 156 rate constants are 99 distinct expressions, 11 of them plain
 Two things bound this kernel and shape the code:
 
   instruction fetch  Every phase is unrolled, far more than a scheduler's instruction cache,
-      so an SM streams its code once per step attempt: about 6 cycles per instruction beyond
-      128 KB of code, however many warps run the same lines at the same time.  Fewer
-      instructions are faster, whatever they do.
+      so an SM streams its code once per step attempt: 6 to 12 cycles per instruction beyond
+      128 KB of code, by how far the warps run together.  Fewer instructions are faster,
+      whatever they do.
   memory latency     A warp has no neighbour on its scheduler to hide behind.  Global loads
       are therefore issued a fixed distance (in emitted operations) before their value is
       used, and each group of tensor-memory loads while the previous group is being used.
@@ -64,6 +64,7 @@ class Stream:
         self.col, self.run_of = w.col, w.run_of
         self.ops = []
         self.names = []
+        self.under_way = set()  # slots with a tensor-memory store not waited for yet
 
     def code(self, text, cost=1):
         self.ops.append(("code", text, cost))
@@ -83,7 +84,7 @@ class Stream:
             self.ops.append(("tload", part))
 
     def tstore(self, pairs):
-        """pairs [(slot, value)] in slot order; waited for at once, so later loads see them."""
+        """pairs [(slot, value)] in slot order; waited for before the next load of one of them."""
         if pairs:
             self.ops.append(("tstore", pairs))
 
@@ -132,6 +133,8 @@ class Stream:
         decl = []
         for i in range(0, len(self.names), 12):
             decl.append("double %s;\n" % ", ".join(self.names[i:i + 12]))
+        if self.under_way:
+            out.append("TST_WAIT;\n")
         regs = sorted({v for o in self.ops if o[0] == "tload" for _, v in o[1]})
         for i in range(0, len(regs), 8):
             decl.append("unsigned %s;\n" % ", ".join("%s_l, %s_h" % (v, v) for v in regs[i:i + 8]))
@@ -139,6 +142,9 @@ class Stream:
 
     def t_issue(self, pairs):
         var, lines, seen = dict(pairs), [], set()
+        if any(x in self.under_way for s0, _ in pairs for x in self.run_of[s0]):
+            lines.append("TST_WAIT;\n")
+            self.under_way.clear()
         for s0, _ in pairs:
             run = self.run_of[s0]
             if run[0] in seen:
@@ -169,7 +175,8 @@ class Stream:
                 i += w
                 if part[0] in val:
                     lines.append("TST%d(%d, %s);\n" % (w, self.col[part[0]], ", ".join(val[s] for s in part)))
-        return lines + ["TST_WAIT;\n"]
+        self.under_way.update(val)
+        return lines
 
 
 class Wide:
