@@ -92,7 +92,8 @@ struct SolveArgs {
     int ld;                  // leading dimension of the struct-of-arrays cell arrays
     double *var;             // [NVAR][ld] species, in/out
     const double *fix;       // [NFIX][ld] H2O, M
-    const double *rconst;    // [NREACT][ld]
+    const double *rconst;    // [NREACT][ld], or with rc_words [distinct constants][ld]
+    int rc_words;            // wide solver: rconst holds one row per distinct constant
     const double *h0;        // optional per-cell starting step
     const int *order;        // optional cell permutation (persistent schedule)
     int *queue;              // work counter (persistent schedule)

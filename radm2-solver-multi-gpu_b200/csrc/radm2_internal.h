@@ -26,6 +26,9 @@ void add_step_counters(int *IPAR, long long nacc, long long nrej, long long nfai
 
 cudaError_t launch_rconst(int n, int ld, const double *jv, const double *temp, const double *fix,
                           const double *rcn2o5, double *rconst, cudaStream_t st);
+// Only the wide solver's distinct constants, one row per word (SolveArgs::rc_words).
+cudaError_t launch_rconst_wide(int n, int ld, const double *jv, const double *temp, const double *fix,
+                               const double *rcn2o5, double *rconst, cudaStream_t st);
 cudaError_t launch_aos_to_soa(int n, int m, int ld, const double *aos, double *soa, cudaStream_t st);
 cudaError_t launch_soa_to_aos(int n, int m, int ld, const double *soa, double *aos, cudaStream_t st);
 // WRF field dimensions (i fastest) and the converted window; mirrors radm2_wrf_grid.

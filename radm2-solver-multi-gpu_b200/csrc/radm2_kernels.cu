@@ -3,6 +3,7 @@
 // per-cell outcomes into the IPAR/RPAR aggregates.
 #include "radm2_device.cuh"
 #include "radm2_internal.h"
+#include "gen/radm2_wide_map.h"
 #include "gen/radm2_wrf.h"
 
 namespace radm2 {
@@ -21,6 +22,34 @@ __global__ void __launch_bounds__(128) k_rconst(int n, int ld, const double *__r
     const double RC_N2O5 = rcn2o5 ? rcn2o5[c] : 0.0;
 #define JV(k) jv[(size_t)(k) * ld + c]
 #define RC_OUT(r, e) rconst[(size_t)(r) * ld + c] = (e)
+#include "gen/radm2_rconst.inc"
+#undef RC_OUT
+#undef JV
+}
+
+// The word of the wide solver that holds reaction r's constant, or -1 when another reaction's
+// word or a number in the code stands for it.
+__host__ __device__ constexpr int wide_rc_word(int r)
+{
+    constexpr int rep[RADM2_WIDE_RC_WORDS] = RADM2_WIDE_RC_REP_INIT;
+    for (int k = 0; k < RADM2_WIDE_RC_WORDS; k++)
+        if (rep[k] == r) return k;
+    return -1;
+}
+
+// k_rconst for the wide solver alone: only its RADM2_WIDE_RC_WORDS distinct constants are
+// formed and stored, row k for word k (the same expressions, so the same values).
+__global__ void __launch_bounds__(128) k_rconst_wide(int n, int ld, const double *__restrict__ jv,
+                                                     const double *__restrict__ temp, const double *__restrict__ fix,
+                                                     const double *__restrict__ rcn2o5, double *__restrict__ rconst)
+{
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= n) return;
+    const double TEMP = temp[c];
+    const double C_M = fix[(size_t)ld + c];
+    const double RC_N2O5 = rcn2o5 ? rcn2o5[c] : 0.0;
+#define JV(k) jv[(size_t)(k) * ld + c]
+#define RC_OUT(r, e) if constexpr (wide_rc_word(r) >= 0) rconst[(size_t)wide_rc_word(r) * ld + c] = (e)
 #include "gen/radm2_rconst.inc"
 #undef RC_OUT
 #undef JV
@@ -241,6 +270,14 @@ cudaError_t launch_rconst(int n, int ld, const double *jv, const double *temp, c
 {
     (void)cudaGetLastError();
     k_rconst<<<(n + 127) / 128, 128, 0, st>>>(n, ld, jv, temp, fix, rcn2o5, rconst);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_rconst_wide(int n, int ld, const double *jv, const double *temp, const double *fix,
+                               const double *rcn2o5, double *rconst, cudaStream_t st)
+{
+    (void)cudaGetLastError();
+    k_rconst_wide<<<(n + 127) / 128, 128, 0, st>>>(n, ld, jv, temp, fix, rcn2o5, rconst);
     return cudaGetLastError();
 }
 

@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(WIDE_BS, 1) k_rosenbrock_wide(const SolveArgs 
 #pragma unroll 8
         for (int k = 0; k < RADM2_WIDE_RC_WORDS; k++)
             asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(sa + (NVAR + k) * (WIDE_BS * 8)),
-                         "l"(rc + (size_t)c_wide_rc_rep[k] * ld)
+                         "l"(rc + (size_t)(a.rc_words ? k : c_wide_rc_rep[k]) * ld)
                          : "memory");
         fix0 = a.fix[cidx];
         fix1 = a.fix[(size_t)ld + cidx];
