@@ -312,7 +312,9 @@ int launch_geometry(radm2_ctx *c, int *bs_out, int *grid_out, size_t *scratch_ou
         grid = c->nsm * info.blocks_per_sm;
         const int need = (c->ncell + 31) / 32;
         if (grid > need) grid = need;
-    } else if (c->o.schedule == RADM2_SCHED_PERSISTENT || wide_solver(c)) {
+    } else if (wide_solver(c)) {
+        grid = wide_shape(c->ncell, c->nsm).grid;
+    } else if (c->o.schedule == RADM2_SCHED_PERSISTENT) {
         int bpsm = c->o.blocks_per_sm > 0 ? c->o.blocks_per_sm : info.blocks_per_sm;
         if (bpsm > info.blocks_per_sm) bpsm = info.blocks_per_sm;
         grid = c->nsm * bpsm;
@@ -364,6 +366,7 @@ SolveArgs make_args(radm2_ctx *c, const SolveParams &p, int *queue)
     a.texit = c->texit;
     a.refine = c->o.refine_sweeps;
     a.coop_selftest = c->coop_selftest;
+    a.warps = wide_solver(c) ? wide_shape(c->ncell, c->nsm).warps : 0;
     return a;
 }
 
@@ -857,7 +860,11 @@ int radm2_rosenbrock_host(radm2_ctx *c, int ncell, double *VAR, const double *FI
         int kg = grid;
         const int cpb = bs * (c->o.cells_per_thread == 2 ? 2 : 1);
         if (c->o.schedule == RADM2_SCHED_COOP) kg = std::min(grid, (m + 31) / 32);
-        else if (c->o.schedule == RADM2_SCHED_PERSISTENT || wide_solver(c)) kg = std::min(grid, (m + cpb - 1) / cpb);
+        else if (wide_solver(c)) {  // the chunk's own shape: never more blocks than the scratch has slots
+            const WideShape ws = wide_shape(m, grid);
+            kg = ws.grid;
+            a.warps = ws.warps;
+        } else if (c->o.schedule == RADM2_SCHED_PERSISTENT) kg = std::min(grid, (m + cpb - 1) / cpb);
         else kg = (m + cpb - 1) / cpb;
         CK(launch_solver(c, a, bs, std::max(kg, 1)));
         CK(launch_reduce(m, c->status + lo, c->nacc + lo, c->nrej + lo, c->texit + lo, c->hexit + lo, c->partials,

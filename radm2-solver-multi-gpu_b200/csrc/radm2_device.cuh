@@ -94,6 +94,7 @@ struct SolveArgs {
     const double *fix;       // [NFIX][ld] H2O, M
     const double *rconst;    // [NREACT][ld], or with rc_words [distinct constants][ld]
     int rc_words;            // wide solver: rconst holds one row per distinct constant
+    int warps;               // wide solver: warps of a block that take cells (0: all four)
     const double *h0;        // optional per-cell starting step
     const int *order;        // optional cell permutation (persistent schedule)
     int *queue;              // work counter (persistent schedule)

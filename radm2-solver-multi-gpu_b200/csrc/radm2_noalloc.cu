@@ -120,11 +120,8 @@ extern "C" int radm2_rosenbrock_noalloc(int ncell, int ld, double *var, const do
     const int ierr0 = parse_params(Tstart, Tend, AbsTol, RelTol, RPAR, IPAR, 1, &p, &autonomous);
     if (ierr0 != 1) return ierr0;
     const size_t off_scratch = kOffRconst + rconst_bytes((size_t)ld);
-    int grid = nsm;
     const size_t slots = ((size_t)RADM2_NOALLOC_BYTES - off_scratch) / kSlotBytes;
-    if ((size_t)grid > slots) grid = (int)slots;
-    const int need = (ncell + 127) / 128;
-    if (grid > need) grid = need;
+    const WideShape shape = wide_shape(ncell, slots < (size_t)nsm ? (int)slots : nsm);
 
     unsigned char *area = nullptr;
     if (area_address(device, &area) != cudaSuccess) return RADM2_E_CUDA;
@@ -142,6 +139,7 @@ extern "C" int radm2_rosenbrock_noalloc(int ncell, int ld, double *var, const do
     a.fix = fix;
     a.rconst = rconst;
     a.rc_words = 1;
+    a.warps = shape.warps;
     a.queue = queue;
     a.scratch = reinterpret_cast<double *>(area + off_scratch);
     a.status = status ? status : reinterpret_cast<int *>(area + kOffStatus);
@@ -156,7 +154,7 @@ extern "C" int radm2_rosenbrock_noalloc(int ncell, int ld, double *var, const do
     // every other region is fully rewritten before it is read.
     if (cudaMemsetAsync(queue, 0, sizeof(int), st) != cudaSuccess) return RADM2_E_CUDA;
     if (launch_rconst_wide(ncell, ld, jv, temp, fix, rc_n2o5, rconst, st) != cudaSuccess) return RADM2_E_CUDA;
-    if (launch_solver_wide(a, grid, st) != cudaSuccess) return RADM2_E_CUDA;
+    if (launch_solver_wide(a, shape.grid, st) != cudaSuccess) return RADM2_E_CUDA;
     if (launch_reduce(ncell, a.status, a.nacc, a.nrej, a.texit, a.hexit, area + kOffPartials, d_res, st) !=
         cudaSuccess)
         return RADM2_E_CUDA;

@@ -96,7 +96,8 @@ __global__ void __launch_bounds__(WIDE_BS, 1) k_rosenbrock_wide(const SolveArgs 
 
     // ---- lane state; a lane starts as one whose (absent) cell is done
     int cidx = -1;
-    bool have = true, outer = true, done = true;
+    bool have = a.warps == 0 || (int)threadIdx.x < 32 * a.warps;
+    bool outer = true, done = true;
     double T = 0.0, H = 1.0, fix0 = 0.0, fix1 = 0.0, hfirst = 0.0;
     int rlast = 0, rmore = 0, nacc = 0, nrej = 0, nstp = 0, status = 1;
 
