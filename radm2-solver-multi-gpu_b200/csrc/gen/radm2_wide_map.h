@@ -9,6 +9,8 @@
 #define RADM2_WIDE_RC_REP_INIT {0,1,2,3,4,5,6,7,8,9,10,11,12,13,14,15,16,17,18,19,20,21,22,23,25,26,27,28,29,30,31,32,33,34,35,36,37,38,40,41,42,43,44,45,46,47,48,49,50,51,52,53,54,55,56,57,58,61,62,69,70,71,72,73,76,90,91,96,97,98,100,101,102,103,104,118,119,120,121,122,125,127,131,132,133,134,139,146}
 #define RADM2_WIDE_SMEM_WORDS 226
 #define RADM2_WIDE_GLOBAL_WORDS 501
+#define RADM2_WIDE_GRCP 501   /* division form: 59 more words, the reciprocal pivots */
+#define RADM2_WIDE_GLOBAL_WORDS_DIV 560
 #define RADM2_WIDE_SPIVOT 147   /* the 28 pivots of rows without eliminations, side by side */
 #define RADM2_WIDE_SPIVOTS 28
 #define RADM2_WIDE_GK1 0

@@ -30,15 +30,21 @@
 namespace radm2 {
 
 constexpr int WIDE_BS = 128;
+#if RADM2_WIDE_DIV
+constexpr int WIDE_GLOBAL_WORDS = RADM2_WIDE_GLOBAL_WORDS_DIV;
+#else
 constexpr int WIDE_GLOBAL_WORDS = RADM2_WIDE_GLOBAL_WORDS;
+#endif
 constexpr int WIDE_SMEM_BYTES = RADM2_WIDE_SMEM_WORDS * WIDE_BS * 8;
 static __constant__ unsigned char c_wide_rc_rep[RADM2_WIDE_RC_WORDS] = RADM2_WIDE_RC_REP_INIT;
 
-// num / den without a branch, so that several proceed together: the hardware's reciprocal
-// estimate, Newton's iteration (cubic, then linear), and Markstein's correction of the
-// quotient by its remainder.  Correctly rounded but for rare reciprocals, provided that the
-// operands stay away from the ends of the exponent range; the caller checks that.
-__device__ __forceinline__ double div_newton(double num, double den)
+// Divisions without the branch of the compiler's own, so that several proceed together: the
+// hardware's reciprocal estimate, Newton's iteration (cubic, then linear), and Markstein's
+// correction of the quotient by its remainder.  The result is the correctly rounded quotient
+// provided that operands and result stay away from the ends of the exponent range; the callers
+// check that and take div_exact otherwise.  (300 million error norms and the parity tests: the
+// same bits as num / den.)
+__device__ __forceinline__ double rcp_newton(double den)
 {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(den));
@@ -46,14 +52,39 @@ __device__ __forceinline__ double div_newton(double num, double den)
     e = fma(e, e, e);
     r = fma(e, r, r);
     e = fma(-den, r, 1.0);
-    r = fma(e, r, r);
+    return fma(e, r, r);
+}
+__device__ __forceinline__ double div_markstein(double num, double den, double r)
+{
     const double q = num * r;
     return fma(fma(-den, q, num), r, q);
 }
-// High words of operands that div_newton takes: den in 2^-496 .. 2^496, num below 2^496.
+// High words of operands that the error norm divides this way: den in 2^-496 .. 2^496, num
+// below 2^496.
 constexpr int DIV_NEWTON_TOP = 0x5f000000, DIV_NEWTON_LOW = 0x21000000;
 
 static __device__ __noinline__ double div_exact(double num, double den) { return num / den; }
+
+#if RADM2_WIDE_DIV
+// The pivot divisions of the reference arithmetic: a pivot's reciprocal is formed once and every
+// division by it takes three operations and a check, 10 instructions instead of 20.  The
+// reciprocal is NaN for a pivot outside 2^-100 .. 2^100, so that its quotients fail the check
+// (a quotient outside 2^-800 .. 2^800 and not zero) and are divided exactly.
+__device__ __forceinline__ double rcp_pivot(double u)
+{
+    const unsigned h = (unsigned)__double2hiint(u) & 0x7fffffffu;
+    return h - 0x39b00000u <= 0x46300000u - 0x39b00000u ? rcp_newton(u) : __hiloint2double(0x7ff80000, 0);
+}
+__device__ __forceinline__ double div_pivot(double a, double u, double r)
+{
+    double q = div_markstein(a, u, r);
+    const unsigned h = (unsigned)__double2hiint(q) & 0x7fffffffu;
+    if (h - 0x0df00000u > 0x71f00000u - 0x0df00000u && !(q == 0.0)) q = div_exact(a, u);
+    return q;
+}
+#define DIVR(a, u, r) div_pivot(a, u, r)
+#define RCPR(u) rcp_pivot(u)
+#endif
 
 // Global scratch, word w of the thread (1 KB apart, so every access of a warp is 256 bytes
 // together).  Volatile statements keep the order in which the generated code issues them;
@@ -205,7 +236,9 @@ __global__ void __launch_bounds__(WIDE_BS, 1) k_rosenbrock_wide(const SolveArgs 
         for (int k = 0; k < RADM2_WIDE_SPIVOTS; k++) {
             const double v = SL(RADM2_WIDE_SPIVOT + k);
             LU_PIVOT_CHECK(v);
-#if !RADM2_WIDE_DIV
+#if RADM2_WIDE_DIV
+            GSTI(RADM2_WIDE_GRCP + k, RCPR(v));
+#else
             SL(RADM2_WIDE_SPIVOT + k) = 1.0 / v;
 #endif
         }
@@ -314,13 +347,9 @@ __global__ void __launch_bounds__(WIDE_BS, 1) k_rosenbrock_wide(const SolveArgs 
                     if (in) V(i + j) = ynew;
                 }
                 if (i + U < END) load();
-#if RADM2_WIDE_DIV
-#pragma unroll
-                for (int j = 0; j < U; j++) q[j] = num[j] / den[j];
-#else
 #pragma unroll
                 for (int j = 0; j < U; j++) {
-                    q[j] = div_newton(num[j], den[j]);
+                    q[j] = div_markstein(num[j], den[j], rcp_newton(den[j]));
                     top = max(top, max(__double2hiint(num[j]), __double2hiint(den[j])));
                     low = min(low, __double2hiint(den[j]));
                 }
@@ -328,7 +357,6 @@ __global__ void __launch_bounds__(WIDE_BS, 1) k_rosenbrock_wide(const SolveArgs 
 #pragma unroll
                     for (int j = 0; j < U; j++) q[j] = div_exact(num[j], den[j]);
                 }
-#endif
 #pragma unroll
                 for (int j = 0; j < U; j++) err += q[j];
             }

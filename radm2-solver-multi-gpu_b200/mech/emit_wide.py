@@ -276,6 +276,11 @@ class Wide:
         ns -= 59 + len(self.rc_rep)
         ng -= GLU
         self.nglobal = GLU + ng
+        # the division form's reciprocal pivots, after everything else: first the pivots of rows
+        # without eliminations, in the order of their shared words
+        rows = [self.irow[sl] for sl in self.lone]
+        rows += [k for k in range(self.n) if k not in set(rows)]
+        self.gr = {k: self.nglobal + i for i, k in enumerate(rows)}
         self.smem_words = 59 + len(self.rc_rep) + ns
         self.acc = acc
 
@@ -299,6 +304,8 @@ class Wide:
              "#define RADM2_WIDE_RC_REP_INIT {%s}\n" % ",".join(map(str, self.rc_rep)),
              "#define RADM2_WIDE_SMEM_WORDS %d\n" % self.smem_words,
              "#define RADM2_WIDE_GLOBAL_WORDS %d\n" % self.nglobal,
+             "#define RADM2_WIDE_GRCP %d   /* division form: %d more words, the reciprocal pivots */\n"
+             "#define RADM2_WIDE_GLOBAL_WORDS_DIV %d\n" % (self.nglobal, self.n, self.nglobal + self.n),
              "#define RADM2_WIDE_SPIVOT %d   /* the %d pivots of rows without eliminations, side by side */\n"
              "#define RADM2_WIDE_SPIVOTS %d\n" % (self.sdiag, len(self.lone), len(self.lone)),
              "#define RADM2_WIDE_GK1 %d\n#define RADM2_WIDE_GK2 %d\n#define RADM2_WIDE_GY %d\n" % (GK1, GK2, GY)]
@@ -443,7 +450,7 @@ class Wide:
                 j = ic[kk]
                 ex = self.read_group(s, list(range(d[j], c[j + 1])), "u%d" % k)
                 need(j)
-                s.code("%s = %s %s %s;" % (w[j], w[j], "*" if recip else "/", ex[d[j]]), 1 if recip else 20)
+                self.divide(s, w[j], ex[d[j]], j, "q%d_%d" % (k, j), recip)
                 self.put_slots(s, [(kk, w[j])], only="GS")
                 for jj in range(d[j] + 1, c[j + 1]):
                     t = ic[jj]
@@ -469,10 +476,22 @@ class Wide:
             if not recip and k not in cols:
                 outs = [(sl, v) for sl, v in outs if sl != dk]
             self.put_slots(s, outs)
+            if not recip:
+                s.code("", 9)
+                s.gstore(self.gr[k], "RCPR(%s)" % w[k])
         self.put("lu" + ("_rcp" if recip else ""), s,
                  "In-place pivot-free LU on the fixed fill pattern, mgpu.cu:2746-2779 order, %s.\n"
                  " * A row's slots that no elimination touches stay where they are" %
                  ("the diagonal slots holding 1/U(k,k) on exit" if recip else "pivot divisions"))
+
+    def divide(self, s, var, pivot, j, name, recip):
+        """var /= pivot of row j: by the reciprocal that the diagonal slot holds, or exactly, by pivot
+        and its reciprocal."""
+        if recip:
+            s.code("%s = %s * %s;" % (var, var, pivot))
+        else:
+            s.gload(name, self.gr[j])
+            s.code("%s = DIVR(%s, %s, %s);" % (var, var, pivot, name), 9)
 
     def put_slots(self, s, pairs, only="GST"):
         ts = []
@@ -506,7 +525,7 @@ class Wide:
             ex = self.read_group(s, list(range(d[k], c[k + 1])), "g")
             for sl in range(d[k] + 1, c[k + 1]):
                 s.code("FNMA(X(%d), %s, X(%d));" % (k, ex[sl], ic[sl]), 2 if self.kind[sl] == "S" else 1)
-            s.code("X(%d) = X(%d) %s %s;" % (k, k, "*" if recip else "/", ex[d[k]]), 1 if recip else 12)
+            self.divide(s, "X(%d)" % k, ex[d[k]], k, "q%d" % k, recip)
         self.put("solve" + ("_rcp" if recip else ""), s,
                  "X = (LU)^-1 X in place, mgpu.cu:2873-3090 order%s" % (", diagonal slots hold reciprocals" if recip else ""))
 

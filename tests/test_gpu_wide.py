@@ -99,3 +99,22 @@ def test_error_norm_beyond_the_branch_free_range(atol):
     assert np.array_equal(out[0][2]["nrej"], out[1][2]["nrej"])
     if atol < 1.0e100:
         assert rel_err(out[0][1], out[1][1]).max() <= SAME_ARITH
+
+
+@pytest.mark.parametrize("h", [1.0e-40, 1.0e-6, 600.0, 1.0e40])
+def test_pivot_divisions_over_the_exponent_range(h):
+    """Reference arithmetic divides by a pivot through its reciprocal; steps that put the pivots
+    1 / (h gamma) outside 2^-100 .. 2^100 (and zero multipliers, at night) take the plain division.
+    Bit for bit the global-scratch kernel of the same arithmetic."""
+    cells = inputs.make_cells(130, 17, "mixed", 0.5)
+    out = []
+    for block in (0, 128):
+        with radm2b200.Solver(parity=1, block_threads=block) as s:
+            s.set_cells(cells)
+            ipar, rpar = radm2b200.default_params(hstart=h, max_steps=6)
+            rpar[0] = min(h, 1.0e-30)
+            ierr = s.rosenbrock(0.0, max(h, 600.0), ATOL, RTOL, rpar, ipar)
+            out.append((ierr, s.get_state(), s.cell_stats()))
+    assert out[0][0] == out[1][0]
+    assert np.array_equal(out[0][1], out[1][1], equal_nan=True)
+    assert all(np.array_equal(out[0][2][k], out[1][2][k], equal_nan=True) for k in out[0][2])

@@ -34,7 +34,7 @@ def harness():
 #include <cstring>
 #include <vector>
 #include "radm2_wide_map.h"
-static double S[RADM2_WIDE_SMEM_WORDS], Gm[RADM2_WIDE_GLOBAL_WORDS], Tm[256], x[59];
+static double S[RADM2_WIDE_SMEM_WORDS], Gm[RADM2_WIDE_GLOBAL_WORDS_DIV], Tm[256], x[59];
 static bool under_way[256];
 static int errors;
 struct Load { unsigned *l, *h; double v; };
@@ -64,6 +64,8 @@ static void tst(int c, double v)
 #define GLD(v, w) v = Gm[w]
 #define GST(w, v) Gm[w] = (v)
 #define LU_PIVOT_CHECK(v) sing |= (v) == 0.0
+#define RCPR(u) (1.0 / (u))
+#define DIVR(a, u, r) ((u) == (u) && (r) != 1.0 / (u) ? (errors++, 0.0) : (a) / (u))
 #define FNMA(c, a, b) c = c - (a) * (b)
 #define FMAC(c, a, b) c = c + (a) * (b)
 ''']
@@ -91,7 +93,7 @@ int jac(const double *fix, double ghinv) {
 int solve%s() {
 #include "radm2_wide_solve%s.inc"
     return errors; }
-''' % (form, "v = 1.0 / v;" if form else "", form, form, form))
+''' % (form, "v = 1.0 / v;" if form else "Gm[RADM2_WIDE_GRCP + k] = 1.0 / v;", form, form, form))
     # the plain reciprocal fragments on an array of slots, for the reciprocal forms
     lines.append('''
 #undef LU_PIVOT_CHECK
@@ -128,7 +130,7 @@ def wide():
 
 class Words:
     def __init__(self, lib, wide):
-        size = {0: wide.smem_words, 1: wide.nglobal, 2: 256, 3: 59}
+        size = {0: wide.smem_words, 1: wide.nglobal + 59, 2: 256, 3: 59}
         self.s, self.g, self.t, self.x = (np.ctypeslib.as_array(lib.words(i), (size[i],)) for i in range(4))
         self.wide = wide
 
