@@ -576,6 +576,13 @@ int radm2_destroy(radm2_ctx *c)
     cudaFree(c->seed_x);
     cudaFree(c->seed_y);
     if (c->mlp) radm2::mlp_detach(c->mlp);
+    for (radm2_ctx::Lane &l : c->lane) {
+        if (l.st) cudaStreamSynchronize(l.st);
+        cudaFree(l.scratch);
+        cudaFree(l.partials);
+        if (l.ev) cudaEventDestroy(l.ev);
+        if (l.st) cudaStreamDestroy(l.st);
+    }
     if (c->scratch) cudaFree(c->scratch);
     if (c->stage) cudaFree(c->stage);
     if (c->partials) cudaFree(c->partials);
@@ -764,11 +771,46 @@ int radm2_rosenbrock(radm2_ctx *c, double Tstart, double Tend, const double *Abs
     return finish(c, 1, autonomous, RPAR, IPAR, p.direction);
 }
 
+// How many compute streams the pipelined host path gets: the context's own and, where its stream,
+// scratch and partial sums can be had, the second.
+static int ensure_lanes(radm2_ctx *c, int nchunk, size_t scratch_bytes)
+{
+    int n = 1;
+    for (; n < std::min(nchunk, (int)radm2_ctx::LANES); n++) {
+        radm2_ctx::Lane &l = c->lane[n];
+        bool ok = (l.st || cudaStreamCreateWithFlags(&l.st, cudaStreamNonBlocking) == cudaSuccess) &&
+                  (l.ev || cudaEventCreateWithFlags(&l.ev, cudaEventDisableTiming) == cudaSuccess) &&
+                  (l.partials || cudaMalloc(&l.partials, reduce_partials_bytes()) == cudaSuccess);
+        if (ok && scratch_bytes > l.scratch_bytes) {
+            cudaFree(l.scratch);
+            l.scratch = nullptr;
+            l.scratch_bytes = 0;
+            ok = cudaMalloc((void **)&l.scratch, scratch_bytes) == cudaSuccess;
+            if (ok) l.scratch_bytes = scratch_bytes;
+        }
+        if (!ok) {
+            (void)cudaGetLastError();
+            break;
+        }
+    }
+    return n;
+}
+
 // Host-buffer integration with the transfers hidden behind the solve: the batch is cut into
 // nchunk consecutive chunks.  Chunk k's inputs go up (copy stream, then a transpose to the
 // struct-of-arrays arrays) while chunk k-1 integrates (rate constants, optional seeding,
 // solver, statistics on the context's stream) and chunk k-2's states come back (transpose
 // and copy on a second copy stream).  Events order each chunk's three steps.
+//
+// With the wide solver, whose blocks fill an SM each, odd chunks go to a second compute stream: a
+// chunk's blocks start on the SMs that the previous chunk's last cells leave, so most of a tail of
+// slow cells costs no time.  200,003 seeded cells in 8 chunks: 86.8 against 95.3 ms on one stream;
+// spun up, 9.6 against 14.3; 1,000,003 spun-up cells in 8 chunks 26.9 against 30.5.  Large chunks
+// lose by it, for the tail is a small share of them and the chunk ahead finishes later, which holds
+// its download back: 1,000,003 cells in 4 chunks 31.8 against 30.1, 200,003 seeded in 2 chunks 74.5
+// against 68.6.  So two streams serve three chunks or more of at most ten cells per lane on average.
+// Four streams were no better (seeded, 8 chunks: 89.3).  The other kernels keep several blocks per
+// SM and two of them compete for it: 1-2% slower, so they stay on one stream.
 int radm2_rosenbrock_host(radm2_ctx *c, int ncell, double *VAR, const double *FIX, const double *TEMP,
                           const double *RC_N2O5, const double *JV, double Tstart, double Tend, const double *AbsTol,
                           const double *RelTol, double *RPAR, int *IPAR, int nchunk)
@@ -806,6 +848,24 @@ int radm2_rosenbrock_host(radm2_ctx *c, int ncell, double *VAR, const double *FI
     }
     const bool order_was = c->use_order;
     c->use_order = false;  // a chunk's cells are integrated in index order
+    const bool spread = wide_solver(c) && nchunk >= 3 && ncell / nchunk <= 10 * 128 * c->nsm;
+    const int lanes = spread ? ensure_lanes(c, nchunk, sbytes) : 1;
+    if (lanes > 1) {  // behind what the caller has put on the context's stream
+        CK(cudaEventRecord(c->lane[1].ev, c->st));
+        for (int l = 1; l < lanes; l++) CK(cudaStreamWaitEvent(c->lane[l].st, c->lane[1].ev, 0));
+    }
+    struct StreamGuard {  // the context's stream again, behind the others, however the call ends
+        radm2_ctx *c;
+        cudaStream_t st;
+        int lanes;
+        ~StreamGuard()
+        {
+            c->st = st;
+            for (int l = 1; l < lanes; l++)
+                if (cudaEventRecord(c->lane[l].ev, c->lane[l].st) == cudaSuccess)
+                    cudaStreamWaitEvent(st, c->lane[l].ev, 0);
+        }
+    } guard{c, c->st, lanes};
     const double dt = std::fabs(p.Tend - p.Tstart);
     // Chunk sizes: with three or more chunks the first and the last are a fifth of a middle
     // one.  Only the first chunk's upload and the last chunk's download are not hidden
@@ -840,12 +900,15 @@ int radm2_rosenbrock_host(radm2_ctx *c, int ncell, double *VAR, const double *FI
         CK(launch_aos_to_soa(m, NPH, c->ld, sj + l * NPH, c->jv + lo, c->st_up));
         CK(cudaEventRecord(c->pipe_ev[2 * k], c->st_up));
         // integrate the chunk
+        const radm2_ctx::Lane &ln = c->lane[k % lanes];
+        c->st = ln.st ? ln.st : guard.st;
         CK(cudaStreamWaitEvent(c->st, c->pipe_ev[2 * k], 0));
         CK(launch_rconst(m, c->ld, c->jv + lo, c->temp + lo, c->fix + lo, RC_N2O5 ? c->rcn + lo : nullptr,
                          c->rconst + lo, c->st));
         if (c->mlp) CK(mlp_enqueue_seed(c, c->mlp, dt, 0, lo, m));
         CK(cudaMemsetAsync(c->queue + k, 0, sizeof(int), c->st));
         SolveArgs a = make_args(c, p, c->queue + k);
+        if (ln.st) a.scratch = ln.scratch;
         a.ncell = m;
         a.var += lo;
         a.fix += lo;
@@ -867,8 +930,8 @@ int radm2_rosenbrock_host(radm2_ctx *c, int ncell, double *VAR, const double *FI
         } else if (c->o.schedule == RADM2_SCHED_PERSISTENT) kg = std::min(grid, (m + cpb - 1) / cpb);
         else kg = (m + cpb - 1) / cpb;
         CK(launch_solver(c, a, bs, std::max(kg, 1)));
-        CK(launch_reduce(m, c->status + lo, c->nacc + lo, c->nrej + lo, c->texit + lo, c->hexit + lo, c->partials,
-                         c->d_res + k, c->st));
+        CK(launch_reduce(m, c->status + lo, c->nacc + lo, c->nrej + lo, c->texit + lo, c->hexit + lo,
+                         ln.st ? ln.partials : c->partials, c->d_res + k, c->st));
         CK(cudaEventRecord(c->pipe_ev[2 * k + 1], c->st));
         // down: this chunk's states
         CK(cudaStreamWaitEvent(c->st_down, c->pipe_ev[2 * k + 1], 0));
@@ -877,6 +940,11 @@ int radm2_rosenbrock_host(radm2_ctx *c, int ncell, double *VAR, const double *FI
                            c->st_down));
     }
     c->use_order = order_was;
+    c->st = guard.st;
+    for (int l = 1; l < lanes; l++) {
+        CK(cudaEventRecord(c->lane[l].ev, c->lane[l].st));
+        CK(cudaStreamWaitEvent(c->st, c->lane[l].ev, 0));
+    }
     CK(cudaMemcpyAsync(c->h_res, c->d_res, sizeof(RunResult) * nchunk, cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
     CK(cudaStreamSynchronize(c->st_down));

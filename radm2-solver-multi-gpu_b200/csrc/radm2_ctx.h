@@ -13,6 +13,16 @@ struct radm2_ctx {
     cudaStream_t own = nullptr;
     cudaStream_t st = nullptr;
     cudaStream_t st_up = nullptr, st_down = nullptr;  // copy streams of the pipelined host path
+    // the pipelined host path's second compute stream, with solver scratch of its own
+    struct Lane {
+        cudaStream_t st = nullptr;
+        cudaEvent_t ev = nullptr;
+        double *scratch = nullptr;
+        size_t scratch_bytes = 0;
+        void *partials = nullptr;
+    };
+    static constexpr int LANES = 2;  // compute streams, the context's own among them
+    Lane lane[LANES];                // lane[0] stays empty: the context's stream and buffers
     std::vector<cudaEvent_t> pipe_ev;                 // per chunk: inputs up, chunk integrated
     int ncell = 0, ld = 0;
     double *var = nullptr, *fix = nullptr, *temp = nullptr, *rcn = nullptr, *jv = nullptr, *rconst = nullptr;

@@ -914,18 +914,19 @@ void radm2::mlp_detach(radm2_mlp *m) { m->attached--; }
 // per-cell h0 (and the descending-cost order when asked).
 cudaError_t radm2::mlp_enqueue_seed(radm2_ctx *c, radm2_mlp *m, double dt, int order, int lo, int count)
 {
-    // cells [lo, lo + count) (count < 0: all); a sub-range gets h0 only, no order
+    // cells [lo, lo + count) (count < 0: all); a sub-range gets h0 only, no order, and its own rows
+    // of the work arrays, as chunks on two streams may be seeded at the same time
     const int n = count < 0 ? c->ncell : count;
     if (count >= 0) order = 0;
+    float *const x = c->seed_x + (size_t)lo * NFEAT, *const y = c->seed_y + (size_t)lo * NY;
     (void)cudaGetLastError();
     k_features<<<(n + FEAT_BLOCK - 1) / FEAT_BLOCK, FEAT_BLOCK, 0, c->st>>>(n, c->ld, c->var + lo, c->fix + lo,
-                                                                         c->temp + lo, c->jv + lo, (float)dt,
-                                                                         c->seed_x);
+                                                                         c->temp + lo, c->jv + lo, (float)dt, x);
     cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = forward(m, n, c->seed_x, c->seed_y, false, c->st);
+    if (e == cudaSuccess) e = forward(m, n, x, y, false, c->st);
     if (e == cudaSuccess) {
-        k_seed<<<(n + 127) / 128, 128, 0, c->st>>>(n, c->seed_y, m->ymean[0], m->ystd[0], m->ymean[1], m->ystd[1],
-                                                   m->h0_scale, c->h0 + lo, c->seed_keys, c->seed_idx);
+        k_seed<<<(n + 127) / 128, 128, 0, c->st>>>(n, y, m->ymean[0], m->ystd[0], m->ymean[1], m->ystd[1], m->h0_scale,
+                                                   c->h0 + lo, c->seed_keys + lo, c->seed_idx + lo);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess && order == 1) {

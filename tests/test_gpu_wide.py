@@ -118,3 +118,24 @@ def test_pivot_divisions_over_the_exponent_range(h):
     assert out[0][0] == out[1][0]
     assert np.array_equal(out[0][1], out[1][1], equal_nan=True)
     assert all(np.array_equal(out[0][2][k], out[1][2][k], equal_nan=True) for k in out[0][2])
+
+
+@pytest.mark.parametrize("nchunk", [2, 3, 8, 17])
+def test_chunks_on_two_streams(nchunk):
+    """Odd chunks run on a second stream with their own scratch, seeded from their own rows of the
+    network's work arrays: bit for bit one chunk's result, call after call."""
+    from radm2b200 import seeding
+    cells = inputs.make_cells(20011, 5, "mixed", 0.4)
+    net = seeding.load_net(seeding.DEFAULT_NET)
+    with radm2b200.Solver(schedule=PERS, placement=WIDE) as s:
+        s.set_cells(cells)
+        s.attach_mlp(net)
+        out = []
+        for k in (1, nchunk, nchunk):
+            y = np.ascontiguousarray(cells["VAR"]).copy()
+            ipar, rpar = radm2b200.default_params(hstart=6.0)
+            assert s.rosenbrock_host(y, cells["FIX"], cells["TEMP"], cells["RC_N2O5"], cells["JV"], 0.0, 600.0, ATOL, RTOL, rpar,
+                                     ipar, nchunk=k) == 1
+            out.append((y, list(ipar[10:17])))
+        s.attach_mlp(None)
+    assert all(np.array_equal(y, out[0][0]) and c == out[0][1] for y, c in out[1:])
