@@ -20,7 +20,7 @@
 //   L2 capacity.  Reads from the scratch run at 12 TB/s while all SMs' scratch stays under
 //   75 MB, 8 TB/s at 100 MB, 4 TB/s at 160 MB (measured).  Per thread: shared memory holds the
 //   state, the 88 distinct rate constants and 79 LU slots, tensor memory 256 LU slots, global
-//   scratch 501 words (74 MB over 148 SMs).
+//   scratch 501 words (76 MB over 148 SMs).
 #pragma once
 
 #include "gen/radm2_wide_map.h"
