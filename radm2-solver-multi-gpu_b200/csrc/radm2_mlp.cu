@@ -18,7 +18,7 @@ namespace radm2 {
 namespace mlp {
 
 constexpr int NIN = 96, NFEAT = 84, W = 128, NOUT = 8, NY = 2;
-constexpr int ROWS = 64;            // samples per CTA
+constexpr int ROWS = 128;           // samples per CTA of the backward kernel (8 warps of 16)
 constexpr int KP_IN = NIN + 8;      // padded k stride (bf16) for the input layer
 constexpr int KP = W + 8;           // padded k stride for hidden layers
 // parameter offsets (floats) in the flat master vector
@@ -39,8 +39,8 @@ constexpr int S_ACT2 = S_ACT + ROWS * KP;    // second activation buffer
 constexpr int S_TOTAL = S_ACT2 + ROWS * KP;  // bf16 elements
 constexpr int SMEM_BYTES = S_TOTAL * 2 + (W * 3 + NOUT) * 4 + NIN * 8;  // + biases + feature norm
 // The forward kernel runs 12 warps per CTA (192 rows per tile) over the one staged weight
-// image: 3x the warps of the training kernels, for latency hiding in the 1-CTA-per-SM
-// footprint (98 KB of weights + 8.7 KB of activations per warp).
+// image, for latency hiding in the 1-CTA-per-SM footprint (98 KB of weights + 8.7 KB of activations per warp).
+static_assert(SMEM_BYTES <= 227 * 1024 && S_ACT % 8 == 0 && KP % 8 == 0 && KP_IN % 8 == 0, "backward kernel shared memory");
 constexpr int FWD_WARPS = 12, FWD_ROWS = FWD_WARPS * 16;
 constexpr int FS_ACT = S_WEND, FS_ACT2 = FS_ACT + FWD_ROWS * KP, FS_TOTAL = FS_ACT2 + FWD_ROWS * KP;
 constexpr int FWD_SMEM_BYTES = FS_TOTAL * 2 + (W * 3 + NOUT) * 4 + NIN * 8;
@@ -197,37 +197,52 @@ __global__ void __launch_bounds__(FWD_WARPS * 32) k_forward(Net net, int n, cons
     }  // tiles
 }
 
-// dW[m][nn] += sum over the warp's 16 rows of A[row][m] * B[row][nn]  (A^T B, K = 16 rows).
-// A rows in smem (stride KA, M columns), B rows in smem (stride KB, NN columns); the
-// products are accumulated into the fp32 gradient (global atomics).
-template <int M, int NN>
-__device__ __forceinline__ void warp_outer(float *grad, int ldg, const __nv_bfloat16 *A, int KA,
-                                           const __nv_bfloat16 *B, int KB, int nvalid)
+// Transposed 8 x 8 blocks of a [k][c] array (row stride K): r0 (k0.., c0..), r1 (k0.., c0 + 8..),
+// r2 (k0 + 8.., c0..), r3 (k0 + 8.., c0 + 8..); a lane gets column c + lane / 4, rows k + 2 (lane % 4), + 1.
+__device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], const __nv_bfloat16 *X, int K, int k0, int c0)
 {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int lane = threadIdx.x & 31;
+    const __nv_bfloat16 *p = X + (k0 + (lane & 7) + ((lane >> 4) & 1) * 8) * K + c0 + ((lane >> 3) & 1) * 8;
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p))
+                 : "memory");
+}
+
+// dW[m][nn] += sum over the CTA's ROWS rows of A[row][m] * B[row][nn]  (A^T B).  A and B rows in
+// smem (stride KP, M and NN columns).  The rows are summed in the tensor cores' FP32 accumulators,
+// and one pair of atomics per element and CTA goes to the gradient: with one per warp of 16 rows
+// (46 million for 16,384 rows) the kernel was bound by the atomics' rate and took 404 us; now 119 us.
+// NN 128: each warp takes 16 columns; NN 8: each warp takes 16 rows of dW.  CTAs start at different
+// rows, so that they do not all add to the same addresses.
+template <int M, int NN>
+__device__ __forceinline__ void block_outer(float *grad, int ldg, const __nv_bfloat16 *A, const __nv_bfloat16 *B,
+                                            int nvalid)
+{
+    static_assert(NN == 128 || (NN == 8 && M == 128), "columns or rows of dW split over 8 warps");
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int c0 = NN == 128 ? warp * 16 : 0;
+    uint32_t b[ROWS / 16][4];
+#pragma unroll
+    for (int kt = 0; kt < ROWS / 16; kt++) ldsm4t(b[kt], B, KP, kt * 16, c0);
 #pragma unroll 1
-    for (int mt = 0; mt < M / 16; mt++) {
-        // A' = A^T: (m, k=row) -> A[row][m]
-        const int m0 = mt * 16 + g, m1 = m0 + 8;
-        const uint32_t a0 = pack2(A + (2 * t) * KA + m0, A + (2 * t + 1) * KA + m0);
-        const uint32_t a1 = pack2(A + (2 * t) * KA + m1, A + (2 * t + 1) * KA + m1);
-        const uint32_t a2 = pack2(A + (2 * t + 8) * KA + m0, A + (2 * t + 9) * KA + m0);
-        const uint32_t a3 = pack2(A + (2 * t + 8) * KA + m1, A + (2 * t + 9) * KA + m1);
-#pragma unroll 4
-        for (int nt = 0; nt < NN / 8; nt++) {
-            const int nn = nt * 8 + g;
-            const uint32_t b0 = pack2(B + (2 * t) * KB + nn, B + (2 * t + 1) * KB + nn);
-            const uint32_t b1 = pack2(B + (2 * t + 8) * KB + nn, B + (2 * t + 9) * KB + nn);
-            float c[4] = {0.f, 0.f, 0.f, 0.f};
-            mma16816(c, a0, a1, a2, a3, b0, b1);
-            const int col = nt * 8 + 2 * t;
+    for (int i = 0; i < (NN == 128 ? M / 16 : 1); i++) {
+        const int mt = NN == 128 ? (i + (int)(blockIdx.x % (M / 16))) % (M / 16) : warp;
+        float c[2][4] = {};
+#pragma unroll
+        for (int kt = 0; kt < ROWS / 16; kt++) {
+            uint32_t a[4];
+            ldsm4t(a, A, KP, kt * 16, mt * 16);
+            mma16816(c[0], a[0], a[1], a[2], a[3], b[kt][0], b[kt][2]);
+            if (NN == 128) mma16816(c[1], a[0], a[1], a[2], a[3], b[kt][1], b[kt][3]);
+        }
+#pragma unroll
+        for (int h = 0; h < (NN == 128 ? 2 : 1); h++) {
+            const int col = c0 + h * 8 + 2 * t;  // even, as are the strides and offsets: 8-byte aligned
             if (col < nvalid) {
-                atomicAdd(&grad[(size_t)(mt * 16 + g) * ldg + col], c[0]);
-                atomicAdd(&grad[(size_t)(mt * 16 + g + 8) * ldg + col], c[2]);
-            }
-            if (col + 1 < nvalid) {
-                atomicAdd(&grad[(size_t)(mt * 16 + g) * ldg + col + 1], c[1]);
-                atomicAdd(&grad[(size_t)(mt * 16 + g + 8) * ldg + col + 1], c[3]);
+                float *d = grad + (size_t)(mt * 16 + g) * ldg + col;
+                atomicAdd(reinterpret_cast<float2 *>(d), make_float2(c[h][0], c[h][1]));
+                atomicAdd(reinterpret_cast<float2 *>(d + 8 * ldg), make_float2(c[h][2], c[h][3]));
             }
         }
     }
@@ -248,12 +263,12 @@ __device__ __forceinline__ void warp_gemm_wt(float (*acc)[4], const __nv_bfloat1
         const uint32_t a2 = ld32(dZ + g * KZ + k0 + 8 + 2 * t);
         const uint32_t a3 = ld32(dZ + (g + 8) * KZ + k0 + 8 + 2 * t);
 #pragma unroll
-        for (int mt = 0; mt < M / 8; mt++) {
+        for (int mt = 0; mt < M / 8; mt += 2) {
             // B(k = j, n = i) = W[i][j] = WT[j][i]
-            const int i = mt * 8 + g;
-            const uint32_t b0 = pack2(WT + (k0 + 2 * t) * KW + i, WT + (k0 + 2 * t + 1) * KW + i);
-            const uint32_t b1 = pack2(WT + (k0 + 2 * t + 8) * KW + i, WT + (k0 + 2 * t + 9) * KW + i);
-            mma16816(acc[mt], a0, a1, a2, a3, b0, b1);
+            uint32_t b[4];
+            ldsm4t(b, WT, KW, k0, mt * 8);
+            mma16816(acc[mt], a0, a1, a2, a3, b[0], b[2]);
+            mma16816(acc[mt + 1], a0, a1, a2, a3, b[1], b[3]);
         }
     }
 }
@@ -538,7 +553,7 @@ __global__ void __launch_bounds__(TC_THREADS) k_forward_tc(Net net, int n, const
 
 // Backward for MSE loss mean over (n x NY): fills grad[NPARAM] (atomic sums over CTAs) and
 // adds the CTA's loss partial to *loss.
-__global__ void __launch_bounds__(128) k_backward(Net net, int n, const float *__restrict__ x,
+__global__ void __launch_bounds__(ROWS * 2) k_backward(Net net, int n, const float *__restrict__ x,
                                                   const float *__restrict__ y, const float *__restrict__ target,
                                                   const float *__restrict__ z1, const float *__restrict__ z2,
                                                   const float *__restrict__ z3, float *__restrict__ grad,
@@ -580,17 +595,22 @@ __global__ void __launch_bounds__(128) k_backward(Net net, int n, const float *_
                 hb[r * KP + k] = __float2bfloat16_rn(v);
             }
         } else {
-            for (int i = lane; i < 16 * W; i += 32) {
-                const int r = i / W, k = i % W, gr = row0 + r;
-                const float v = gr < n ? gelu(zs[l][(size_t)gr * W + k]) : 0.f;
-                hb[r * KP + k] = __float2bfloat16_rn(v);
+            const int k = lane * 4;
+#pragma unroll 8
+            for (int r = 0; r < 16; r++) {
+                uint2 o = make_uint2(0u, 0u);
+                if (row0 + r < n) {
+                    const float4 z = *reinterpret_cast<const float4 *>(zs[l] + (size_t)(row0 + r) * W + k);
+                    o = make_uint2(pack_bf16(gelu(z.x), gelu(z.y)), pack_bf16(gelu(z.z), gelu(z.w)));
+                }
+                *reinterpret_cast<uint2 *>(hb + r * KP + k) = o;
             }
         }
     };
     load_h(2);
-    __syncwarp();
+    __syncthreads();
     // layer 4: dW4 = h3^T dY (128 x 8, 2 valid columns), db4 = sum dY
-    warp_outer<W, NOUT>(grad + OFF_W4, NOUT, hb, KP, db, KP, NY);
+    block_outer<W, NOUT>(grad + OFF_W4, NOUT, sw + S_ACT, sw + S_ACT2, NY);
     if (lane < NY) {
         float s = 0.f;
         for (int r = 0; r < 16; r++) s += __bfloat162float(db[r * KP + lane]);
@@ -617,8 +637,8 @@ __global__ void __launch_bounds__(128) k_backward(Net net, int n, const float *_
     const __nv_bfloat16 *wts[3] = {sw + S_WT1, sw + S_WT2, sw + S_WT3};
 #pragma unroll 1
     for (int l = 2; l >= 0; l--) {
-        __syncwarp();
-        // dZ_l = dH_l * gelu'(z_l) -> db (bf16); db_l bias gradient
+        __syncthreads();  // every warp is done with the rows of the layer above
+        // dZ_l = dH_l * gelu'(z_l) -> db (bf16)
 #pragma unroll
         for (int mt = 0; mt < 16; mt++) {
 #pragma unroll
@@ -626,25 +646,28 @@ __global__ void __launch_bounds__(128) k_backward(Net net, int n, const float *_
                 const int r = g + 8 * h, c = mt * 8 + 2 * t, gr = row0 + r;
                 float d0 = 0.f, d1 = 0.f;
                 if (gr < n) {
-                    d0 = acc[mt][2 * h] * gelu_grad(zs[l][(size_t)gr * W + c]);
-                    d1 = acc[mt][2 * h + 1] * gelu_grad(zs[l][(size_t)gr * W + c + 1]);
+                    const float2 z = *reinterpret_cast<const float2 *>(zs[l] + (size_t)gr * W + c);
+                    d0 = acc[mt][2 * h] * gelu_grad(z.x);
+                    d1 = acc[mt][2 * h + 1] * gelu_grad(z.y);
                 }
                 *reinterpret_cast<uint32_t *>(db + r * KP + c) = pack_bf16(d0, d1);
             }
         }
-        __syncwarp();
-        for (int c = lane; c < W; c += 32) {
+        // h_{l-1} (or the input) -> hb; dW_l = h_{l-1}^T dZ_l, bias gradient = sum dZ_l
+        load_h(l - 1);
+        __syncthreads();
+        {
+            static_assert(ROWS * 2 == 2 * W, "two threads per bias");
+            const int c = threadIdx.x % W, r0 = threadIdx.x / W * (ROWS / 2);
             float s = 0.f;
-            for (int r = 0; r < 16; r++) s += __bfloat162float(db[r * KP + c]);
+#pragma unroll 8
+            for (int r = r0; r < r0 + ROWS / 2; r++) s += __bfloat162float(sw[S_ACT2 + r * KP + c]);
             atomicAdd(&grad[offB[l] + c], s);
         }
-        // h_{l-1} (or the input) -> hb; dW_l = h_{l-1}^T dZ_l
-        load_h(l - 1);
-        __syncwarp();
         if (l == 0)
-            warp_outer<NIN, W>(grad + offW[0], W, hb, KP, db, KP, W);
+            block_outer<NIN, W>(grad + offW[0], W, sw + S_ACT, sw + S_ACT2, W);
         else
-            warp_outer<W, W>(grad + offW[l], W, hb, KP, db, KP, W);
+            block_outer<W, W>(grad + offW[l], W, sw + S_ACT, sw + S_ACT2, W);
         if (l > 0) {
             // dH_{l-1} = dZ_l W_l^T
             warp_gemm_wt<W, W>(acc, db, KP, wts[l], KP);
@@ -861,7 +884,7 @@ cudaError_t backward(radm2_mlp *m, int n, const float *dx, const float *dt)
     const size_t zs = (size_t)m->zcap * W;
     cudaError_t e = cudaMemsetAsync(m->loss, 0, sizeof(float), m->st);
     if (e != cudaSuccess) return e;
-    k_backward<<<(n + ROWS - 1) / ROWS, 128, SMEM_BYTES, m->st>>>(net_of(m), n, dx, m->y, dt, m->z, m->z + zs,
+    k_backward<<<(n + ROWS - 1) / ROWS, ROWS * 2, SMEM_BYTES, m->st>>>(net_of(m), n, dx, m->y, dt, m->z, m->z + zs,
                                                                   m->z + 2 * zs, m->g, m->loss);
     return cudaGetLastError();
 }

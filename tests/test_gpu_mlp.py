@@ -70,6 +70,23 @@ def test_gradients_match_reference(feats):
         assert np.linalg.norm(a - c) <= 1e-1 * np.linalg.norm(c) + 1e-9, name
 
 
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 127, 128, 129, 300])
+def test_gradients_at_tile_edges(feats, n):
+    """Batches around a warp's 16 and a block's 128 rows.  The FP32 sums and the reference's FP64
+    sums may round an upstream gradient to neighbouring bfloat16 values, 2^-8 apart: four layers of
+    that are 1.6e-2 of a tensor's norm at most."""
+    net, xm, xs = _net(feats)
+    t = np.random.default_rng(2).normal(size=(n, 2)).astype(np.float32)
+    g, loss = net.gradients(feats[:n], t)
+    _, loss_r, g_r = mlp_ref.forward_backward(net.params(), xm, xs, feats[:n], t, bf=True)
+    assert abs(loss - loss_r) <= 1e-3 * loss_r
+    o = 0
+    for name, k in mlp_ref.SIZES:
+        a, b = g[o:o + k], g_r[o:o + k]
+        o += k
+        assert np.linalg.norm(a - b) <= 1.6e-2 * np.linalg.norm(b) + 1e-9, name
+
+
 def test_training_reduces_loss_and_gains_steps():
     """Train on traces of one seed, evaluate on a disjoint seed: seeded starting steps must
     cut the step attempts of the same integration.  Accuracy against an FP64 rtol 1e-8
