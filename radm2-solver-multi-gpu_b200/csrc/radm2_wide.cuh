@@ -25,6 +25,7 @@
 
 #include "gen/radm2_wide_map.h"
 #include "gen/radm2_wide_tmem.h"
+#include "radm2_div.cuh"
 #include "radm2_internal.h"
 
 namespace radm2 {
@@ -38,50 +39,7 @@ constexpr int WIDE_GLOBAL_WORDS = RADM2_WIDE_GLOBAL_WORDS;
 constexpr int WIDE_SMEM_BYTES = RADM2_WIDE_SMEM_WORDS * WIDE_BS * 8;
 static __constant__ unsigned char c_wide_rc_rep[RADM2_WIDE_RC_WORDS] = RADM2_WIDE_RC_REP_INIT;
 
-// Divisions without the branch of the compiler's own, so that several proceed together: the
-// hardware's reciprocal estimate, Newton's iteration (cubic, then linear), and Markstein's
-// correction of the quotient by its remainder.  The result is the correctly rounded quotient
-// provided that operands and result stay away from the ends of the exponent range; the callers
-// check that and take div_exact otherwise.  (300 million error norms and the parity tests: the
-// same bits as num / den.)
-__device__ __forceinline__ double rcp_newton(double den)
-{
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(den));
-    double e = fma(-den, r, 1.0);
-    e = fma(e, e, e);
-    r = fma(e, r, r);
-    e = fma(-den, r, 1.0);
-    return fma(e, r, r);
-}
-__device__ __forceinline__ double div_markstein(double num, double den, double r)
-{
-    const double q = num * r;
-    return fma(fma(-den, q, num), r, q);
-}
-// High words of operands that the error norm divides this way: den in 2^-496 .. 2^496, num
-// below 2^496.
-constexpr int DIV_NEWTON_TOP = 0x5f000000, DIV_NEWTON_LOW = 0x21000000;
-
-static __device__ __noinline__ double div_exact(double num, double den) { return num / den; }
-
 #if RADM2_WIDE_DIV
-// The pivot divisions of the reference arithmetic: a pivot's reciprocal is formed once and every
-// division by it takes three operations and a check, 10 instructions instead of 20.  The
-// reciprocal is NaN for a pivot outside 2^-100 .. 2^100, so that its quotients fail the check
-// (a quotient outside 2^-800 .. 2^800 and not zero) and are divided exactly.
-__device__ __forceinline__ double rcp_pivot(double u)
-{
-    const unsigned h = (unsigned)__double2hiint(u) & 0x7fffffffu;
-    return h - 0x39b00000u <= 0x46300000u - 0x39b00000u ? rcp_newton(u) : __hiloint2double(0x7ff80000, 0);
-}
-__device__ __forceinline__ double div_pivot(double a, double u, double r)
-{
-    double q = div_markstein(a, u, r);
-    const unsigned h = (unsigned)__double2hiint(q) & 0x7fffffffu;
-    if (h - 0x0df00000u > 0x71f00000u - 0x0df00000u && !(q == 0.0)) q = div_exact(a, u);
-    return q;
-}
 #define DIVR(a, u, r) div_pivot(a, u, r)
 #define RCPR(u) rcp_pivot(u)
 #endif
@@ -332,8 +290,7 @@ __global__ void __launch_bounds__(WIDE_BS, 1) k_rosenbrock_wide(const SolveArgs 
             load();
 #pragma unroll 1
             for (int i = 0; i < END; i += U) {
-                double num[U], den[U], q[U];
-                int top = 0, low = 0x7fffffff;
+                double num[U], den[U];
 #pragma unroll
                 for (int j = 0; j < U; j++) {
                     const bool in = j < U - (END - NVAR) || i + j < NVAR;  // the last step is not full
@@ -348,17 +305,7 @@ __global__ void __launch_bounds__(WIDE_BS, 1) k_rosenbrock_wide(const SolveArgs 
                 }
                 if (i + U < END) load();
 #pragma unroll
-                for (int j = 0; j < U; j++) {
-                    q[j] = div_markstein(num[j], den[j], rcp_newton(den[j]));
-                    top = max(top, max(__double2hiint(num[j]), __double2hiint(den[j])));
-                    low = min(low, __double2hiint(den[j]));
-                }
-                if (top > DIV_NEWTON_TOP || low < DIV_NEWTON_LOW) {
-#pragma unroll
-                    for (int j = 0; j < U; j++) q[j] = div_exact(num[j], den[j]);
-                }
-#pragma unroll
-                for (int j = 0; j < U; j++) err += q[j];
+                for (int j = 0; j < U; j++) err += num[j] / den[j];
             }
         }
 
