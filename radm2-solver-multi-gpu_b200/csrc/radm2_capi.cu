@@ -230,9 +230,10 @@ int radm2::parse_params(double Tstart, double Tend, const double *AbsTol, const 
     for (int i = 0; i < uplim; i++)
         if ((AbsTol[i] <= 0.0) || (RelTol[i] <= 10.0 * p->Roundoff) || (RelTol[i] >= 1.0)) return -5;
     if (IPAR[3] != 2) return -2;  // only ROS-3 is wired (mgpu.cu:3803-3811)
-    for (int i = 0; i < NVAR; i++) {
-        p->AbsTol[i] = vector_tol ? AbsTol[i] : AbsTol[0];
-        p->RelTol[i] = vector_tol ? RelTol[i] : RelTol[0];
+    for (int i = 0; i < NTOL; i++) {
+        const int k = vector_tol ? std::min(i, NVAR - 1) : 0;
+        p->AbsTol[i] = AbsTol[k];
+        p->RelTol[i] = RelTol[k];
     }
     for (int i = 0; i < 3; i++) {
         p->M[i] = float_coeffs ? (double)(float)ros_M[i] : ros_M[i];

@@ -23,6 +23,7 @@
 namespace radm2 {
 
 constexpr int NVAR = RADM2_NVAR;
+constexpr int NTOL = (NVAR + 3) / 4 * 4;  // tolerances are read four species at a time
 constexpr int NFIX = RADM2_NFIX;
 constexpr int NREACT = RADM2_NREACT;
 constexpr int NJVS = RADM2_LU_NONZERO;
@@ -81,7 +82,7 @@ struct SolveParams {
     double FacMin, FacMax, FacRej, FacSafe;
     double Roundoff;
     double M[3], E[3];  // ROS-3 M and E (float-rounded in reference-parity mode)
-    double AbsTol[NVAR], RelTol[NVAR];
+    double AbsTol[NTOL], RelTol[NTOL];  // beyond NVAR: the last species' again
     int max_steps;      // per-cell attempt cap (>0)
     int direction;      // +1 / -1
 };

@@ -275,7 +275,8 @@ __global__ void __launch_bounds__(WIDE_BS, 1) k_rosenbrock_wide(const SolveArgs 
         double err = 0.0;
         {
             constexpr int U = 4, END = (NVAR + U - 1) / U * U;
-            static_assert(END - NVAR < U && RADM2_WIDE_GY + END <= WIDE_GLOBAL_WORDS, "the last step reads past the species");
+            static_assert(END - NVAR < U && RADM2_WIDE_GY + END <= WIDE_GLOBAL_WORDS && END <= NTOL,
+                          "the last step reads past the species");
             double k0[U], k1[U], y[U];
             const double *g = gp;
             auto load = [&]() {
