@@ -591,6 +591,7 @@ int radm2_destroy(radm2_ctx *c)
     if (c->h_res) cudaFreeHost(c->h_res);
     if (c->queue) cudaFree(c->queue);
     for (cudaEvent_t e : c->pipe_ev) cudaEventDestroy(e);
+    if (c->pipe_start) cudaEventDestroy(c->pipe_start);
     if (c->st_up) cudaStreamDestroy(c->st_up);
     if (c->st_down) cudaStreamDestroy(c->st_down);
     if (c->own) cudaStreamDestroy(c->own);
@@ -847,26 +848,31 @@ int radm2_rosenbrock_host(radm2_ctx *c, int ncell, double *VAR, const double *FI
         CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         c->pipe_ev.push_back(e);
     }
-    const bool order_was = c->use_order;
-    c->use_order = false;  // a chunk's cells are integrated in index order
     const bool spread = wide_solver(c) && nchunk >= 3 && ncell / nchunk <= 10 * 128 * c->nsm;
     const int lanes = spread ? ensure_lanes(c, nchunk, sbytes) : 1;
-    if (lanes > 1) {  // behind what the caller has put on the context's stream
-        CK(cudaEventRecord(c->lane[1].ev, c->st));
-        for (int l = 1; l < lanes; l++) CK(cudaStreamWaitEvent(c->lane[l].st, c->lane[1].ev, 0));
-    }
-    struct StreamGuard {  // the context's stream again, behind the others, however the call ends
+    // Every stream begins behind what is already on the context's: transposes of earlier uploads
+    // read the staging buffer and write the cell arrays that the copy streams fill, and copies of
+    // the state out of them may be under way.
+    if (!c->pipe_start) CK(cudaEventCreateWithFlags(&c->pipe_start, cudaEventDisableTiming));
+    CK(cudaEventRecord(c->pipe_start, c->st));
+    CK(cudaStreamWaitEvent(c->st_up, c->pipe_start, 0));
+    CK(cudaStreamWaitEvent(c->st_down, c->pipe_start, 0));
+    for (int l = 1; l < lanes; l++) CK(cudaStreamWaitEvent(c->lane[l].st, c->pipe_start, 0));
+    // The context's stream again however the call ends; if it ends early, the caller's arrays and the
+    // context's are not in use any more when it returns.
+    struct StreamGuard {
         radm2_ctx *c;
         cudaStream_t st;
         int lanes;
+        bool finished;
         ~StreamGuard()
         {
             c->st = st;
-            for (int l = 1; l < lanes; l++)
-                if (cudaEventRecord(c->lane[l].ev, c->lane[l].st) == cudaSuccess)
-                    cudaStreamWaitEvent(st, c->lane[l].ev, 0);
+            if (finished) return;
+            for (int l = 1; l < lanes; l++) cudaStreamSynchronize(c->lane[l].st);
+            for (cudaStream_t q : {c->st_up, c->st, c->st_down}) cudaStreamSynchronize(q);
         }
-    } guard{c, c->st, lanes};
+    } guard{c, c->st, lanes, false};
     const double dt = std::fabs(p.Tend - p.Tstart);
     // Chunk sizes: with three or more chunks the first and the last are a fifth of a middle
     // one.  Only the first chunk's upload and the last chunk's download are not hidden
@@ -909,6 +915,7 @@ int radm2_rosenbrock_host(radm2_ctx *c, int ncell, double *VAR, const double *FI
         if (c->mlp) CK(mlp_enqueue_seed(c, c->mlp, dt, 0, lo, m));
         CK(cudaMemsetAsync(c->queue + k, 0, sizeof(int), c->st));
         SolveArgs a = make_args(c, p, c->queue + k);
+        a.order = nullptr;  // a chunk's cells are integrated in index order
         if (ln.st) a.scratch = ln.scratch;
         a.ncell = m;
         a.var += lo;
@@ -940,7 +947,6 @@ int radm2_rosenbrock_host(radm2_ctx *c, int ncell, double *VAR, const double *FI
         CK(cudaMemcpyAsync(VAR + l * NVAR, so + l * NVAR, sizeof(double) * m * NVAR, cudaMemcpyDeviceToHost,
                            c->st_down));
     }
-    c->use_order = order_was;
     c->st = guard.st;
     for (int l = 1; l < lanes; l++) {
         CK(cudaEventRecord(c->lane[l].ev, c->lane[l].st));
@@ -950,6 +956,7 @@ int radm2_rosenbrock_host(radm2_ctx *c, int ncell, double *VAR, const double *FI
     CK(cudaStreamSynchronize(c->st));
     CK(cudaStreamSynchronize(c->st_down));
     CK(cudaStreamSynchronize(c->st_up));
+    guard.finished = true;
     // one result over all chunks: counters summed, exit times and steps at their extremes
     RunResult tot = c->h_res[0];
     for (int k = 1; k < nchunk; k++) {

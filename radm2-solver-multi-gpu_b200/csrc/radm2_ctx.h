@@ -13,6 +13,7 @@ struct radm2_ctx {
     cudaStream_t own = nullptr;
     cudaStream_t st = nullptr;
     cudaStream_t st_up = nullptr, st_down = nullptr;  // copy streams of the pipelined host path
+    cudaEvent_t pipe_start = nullptr;                 // what its streams begin behind
     // the pipelined host path's second compute stream, with solver scratch of its own
     struct Lane {
         cudaStream_t st = nullptr;
