@@ -1278,7 +1278,11 @@ int radm2_autotune(radm2_ctx *c, double dt, const double *AbsTol, const double *
     if (e == cudaSuccess) e = launch_gather_rows(n, NPH, c->ld, stride, c->jv, t->ld, t->jv, t->st);
     if (e == cudaSuccess && c->have_rcn) e = launch_gather_rows(n, 1, c->ld, stride, c->rcn, t->ld, t->rcn, t->st);
     t->have_rcn = c->have_rcn;
-    t->rconst_valid = false;
+    // constants set by the caller choose the kernels (wide_solver) and the steps: the sample takes them too
+    t->rconst_valid = c->rconst_valid && !c->rconst_formula;
+    t->rconst_formula = !t->rconst_valid;
+    if (e == cudaSuccess && t->rconst_valid)
+        e = launch_gather_rows(n, NREACT, c->ld, stride, c->rconst, t->ld, t->rconst, t->st);
     if (e == cudaSuccess) e = cudaMalloc((void **)&y0, sizeof(double) * NVAR * t->ld);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(y0, t->var, sizeof(double) * NVAR * t->ld, cudaMemcpyDeviceToDevice, t->st);
