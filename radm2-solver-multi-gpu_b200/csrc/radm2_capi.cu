@@ -1396,7 +1396,9 @@ int radm2_autotune(radm2_ctx *c, double dt, const double *AbsTol, const double *
 size_t radm2_device_bytes(const radm2_ctx *c)
 {
     if (!c) return 0;
-    return c->bytes + c->scratch_bytes + c->stage_bytes;
+    size_t n = c->bytes + c->scratch_bytes + c->stage_bytes;
+    for (const radm2_ctx::Lane &l : c->lane) n += l.scratch_bytes + (l.partials ? reduce_partials_bytes() : 0);
+    return n;
 }
 
 int radm2_coop_selftest_wait_limit(radm2_ctx *c)

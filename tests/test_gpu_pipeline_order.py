@@ -50,3 +50,18 @@ def test_host_call_leaves_the_visiting_order():
         s.set_cell_order(order)
         got = host_call(s, cells, 5)
     assert np.array_equal(got[0], want[0]) and got[1] == want[1]
+
+
+def test_device_bytes_count_the_second_stream():
+    """The second compute stream's scratch is the context's: radm2_device_bytes grows by what the
+    device loses."""
+    torch = pytest.importorskip("torch")
+    cells = inputs.make_cells(20000, 8, "plain", 0.3)
+    with radm2b200.Solver() as s:
+        host_call(s, cells, 1)
+        held, free = s.device_bytes(), torch.cuda.mem_get_info()[0]
+        host_call(s, cells, 8)
+        grown, lost = s.device_bytes() - held, free - torch.cuda.mem_get_info()[0]
+        assert grown > 32 << 20 and abs(lost - grown) <= 8 << 20  # allocations come in pages of 2 MiB
+        host_call(s, cells, 8)
+        assert s.device_bytes() - held == grown
