@@ -806,13 +806,22 @@ static int ensure_lanes(radm2_ctx *c, int nchunk, size_t scratch_bytes)
 //
 // With the wide solver, whose blocks fill an SM each, odd chunks go to a second compute stream: a
 // chunk's blocks start on the SMs that the previous chunk's last cells leave, so most of a tail of
-// slow cells costs no time.  200,003 seeded cells in 8 chunks: 86.8 against 95.3 ms on one stream;
-// spun up, 9.6 against 14.3; 1,000,003 spun-up cells in 8 chunks 26.9 against 30.5.  Large chunks
-// lose by it, for the tail is a small share of them and the chunk ahead finishes later, which holds
-// its download back: 1,000,003 cells in 4 chunks 31.8 against 30.1, 200,003 seeded in 2 chunks 74.5
-// against 68.6.  So two streams serve three chunks or more of at most ten cells per lane on average.
-// Four streams were no better (seeded, 8 chunks: 89.3).  The other kernels keep several blocks per
-// SM and two of them compete for it: 1-2% slower, so they stay on one stream.
+// slow cells costs no time.  Large chunks lose by it, for the tail is a small share of them and the
+// chunk ahead finishes later, which holds its download back.  Measured (ms on one stream / on two), by
+// cells per lane of an average chunk (148 SMs x 128 lanes), from the cold start and spun up, seeded:
+//   0.1  20,011 cells, 8 chunks   51.0 / 30.2   and   8.0 /  4.5
+//   0.4  65,539 cells, 8          54.1 / 36.9   and   9.9 /  5.5
+//   1.3  200,003 cells, 8         94.1 / 82.8   and  14.2 /  9.4
+//   2.6  200,003 cells, 4         69.5 / 68.7   and  10.1 /  8.1
+//   3.5  200,003 cells, 3         69.2 / 70.6   and   8.9 /  8.5
+//   5.3  400,009 cells, 4        141.7 / 134.5  and  14.5 / 13.7
+//   7.0  400,009 cells, 3        137.6 / 128.6  and  14.9 / 15.5
+//   9.2  700,001 cells, 4                            22.0 / 22.9
+//   12   700,001 cells, 3                            25.3 / 25.7
+// So two streams serve three chunks or more of at most six cells per lane on average; two chunks gain
+// nothing (200,003 seeded cells 74.5 ms, 68.6 on one stream).  Four streams were no better (200,003
+// seeded cells in 8 chunks: 89.3 ms, 86.8 with two).  The other kernels keep several blocks per SM
+// and two of them compete for it: 1-2% slower, so they stay on one stream.
 int radm2_rosenbrock_host(radm2_ctx *c, int ncell, double *VAR, const double *FIX, const double *TEMP,
                           const double *RC_N2O5, const double *JV, double Tstart, double Tend, const double *AbsTol,
                           const double *RelTol, double *RPAR, int *IPAR, int nchunk)
@@ -848,7 +857,7 @@ int radm2_rosenbrock_host(radm2_ctx *c, int ncell, double *VAR, const double *FI
         CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         c->pipe_ev.push_back(e);
     }
-    const bool spread = wide_solver(c) && nchunk >= 3 && ncell / nchunk <= 10 * 128 * c->nsm;
+    const bool spread = wide_solver(c) && nchunk >= 3 && ncell / nchunk <= 6 * 128 * c->nsm;
     const int lanes = spread ? ensure_lanes(c, nchunk, sbytes) : 1;
     // Every stream begins behind what is already on the context's: transposes of earlier uploads
     // read the staging buffer and write the cell arrays that the copy streams fill, and copies of
