@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "../../include/radm2.h"
+#include "gen/radm2_wide_map.h"
 #include "radm2_internal.h"
 
 namespace radm2 {
@@ -310,6 +311,7 @@ constexpr long long TC_WAIT_CYCLES = 4000000000LL;  // and SM cycles (~2 s): a t
                                                     // may suspend for a hardware-defined time
 static_assert(TB_ACT % 16 == 0 && TB_W2 % 16 == 0 && TB_W4 % 16 == 0 && TB_MBAR % 8 == 0, "operand alignment");
 static_assert(TC_SMEM <= 227 * 1024, "tcgen05 forward shared memory");
+static_assert(TC_SMEM + RADM2_WIDE_SMEM_WORDS * 128 * 8 > 228 * 1024, "an SM holds this kernel's CTA or the wide solver's");
 static_assert(TC_TMEM_COLS <= 512, "tensor memory columns");
 static_assert(NFEAT % 4 == 0 && NIN % 8 == 0, "feature rows in 16-byte groups");
 
@@ -438,8 +440,9 @@ __global__ void __launch_bounds__(TC_THREADS) k_forward_tc(Net net, int n, const
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(mbar) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
-    // one warp owns the tensor-memory allocation; the shared-memory footprint keeps one CTA
-    // per SM and no other kernel of the library uses tensor memory, so the 512 columns are free
+    // One warp owns the tensor-memory allocation.  The shared-memory footprint keeps one CTA per SM
+    // and the wide solver, which takes all 512 columns and may run on another stream, off that SM; a
+    // solver with 128 slots may share it, and the allocation then waits until its CTAs are done.
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(sbase + TB_TMEM),
                      "r"(TC_TMEM_COLS)

@@ -32,7 +32,7 @@ constexpr size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 
 // Offsets of the carved regions (bytes): the per-cell bookkeeping, then the rate constants of the
 // call's cells (only the wide solver's distinct ones), and the rest for the solver's scratch, one
-// slot per block: 111 blocks for 10,000 cells, 80 for the largest batch.
+// slot per block: 114 slots at 10,000 cells (which take 105 blocks), 83 for the largest batch.
 constexpr int kMinBlocks = 64;
 constexpr size_t kCells = RADM2_NOALLOC_MAX_CELLS;
 constexpr size_t kOffNacc = 0;
