@@ -269,8 +269,9 @@ __global__ void __launch_bounds__(WIDE_BS, 1) k_rosenbrock_wide(const SolveArgs 
         }
 
         // New state (into V) and error norm (mgpu.cu:3223-3238), U species at a time, the next
-        // ones' K1, K2 and state being loaded meanwhile.  The sum is in species order.  The plain
-        // divisions follow one another, 141 cycles each: 3-4% of the kernel.
+        // ones' K1, K2 and state being loaded meanwhile.  The sum is in species order.  A
+        // division takes 141 cycles and they follow one another, so four species share one
+        // (262,144 cells x 2 steps 116.5 ms, 119.2 with one each).
 #pragma unroll
         for (int i = 0; i < NVAR; i++) V(i) = x[i];  // K3
         double err = 0.0;
@@ -292,8 +293,7 @@ __global__ void __launch_bounds__(WIDE_BS, 1) k_rosenbrock_wide(const SolveArgs 
             load();
 #pragma unroll 1
             for (int i = 0; i < END; i += U) {
-                double num[U], den[U];
-                bool none[U];
+                double num[U], den[U], q[U];
 #pragma unroll
                 for (int j = 0; j < U; j++) {
                     const bool in = j < U - (END - NVAR) || i + j < NVAR;  // the last step is not full
@@ -302,20 +302,14 @@ __global__ void __launch_bounds__(WIDE_BS, 1) k_rosenbrock_wide(const SolveArgs 
                     const double yerr = P.E[0] * k0[j] + P.E[1] * k1[j] + P.E[2] * k2;
                     const double ymax = maxd(fabs(y[j]), fabs(ynew));
                     const double scale = P.AbsTol[i + j] + P.RelTol[i + j] * ymax;
-                    num[j] = yerr * yerr;
+                    num[j] = in ? yerr * yerr : 0.0;
                     den[j] = in ? scale * scale : 1.0;
-                    // A zero numerator takes the division's slow path, and one lane is enough: one
-                    // cell in a warp 4.8 ms a step, 3.9 with 1 / den computed and dropped instead.
-                    none[j] = !in || (num[j] == 0.0 && den[j] > 1e-150 && den[j] < 1e150);
-                    if (none[j]) num[j] = 1.0;
                     if (in) V(i + j) = ynew;
                 }
                 if (i + U < END) load();
+                div_four(num, den, q);
 #pragma unroll
-                for (int j = 0; j < U; j++) {
-                    const double q = num[j] / den[j];
-                    err += none[j] ? 0.0 : q;
-                }
+                for (int j = 0; j < U; j++) err += q[j];
             }
         }
 
