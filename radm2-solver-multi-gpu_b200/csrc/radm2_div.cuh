@@ -16,36 +16,37 @@ static __device__ __noinline__ double div_exact(double a, double u) { return a /
 // exact remainder, hence operands and quotient away from the ends of the exponent range.
 //
 // Operands: any.  Zeros keep their sign; what could leave the range is divided plainly.  The wide
-// solver in reference arithmetic, 8,191 cells of one step: 12.5 ms, 19.5 with a / u throughout.
+// solver in reference arithmetic, 8,191 cells of one step: 12.1 ms, 19.5 with a / u throughout.
 
-// The reciprocal for div_pivot: NaN for a pivot outside 2^-100 .. 2^100, whose quotients then fail
-// div_pivot's check.
+// The reciprocal for div_pivot: NaN for a pivot that is negative (backward integration, negative
+// states) or outside 2^-100 .. 2^100; its quotients are divided plainly.
 __device__ __forceinline__ double rcp_pivot(double u)
 {
-    const unsigned h = (unsigned)__double2hiint(u) & 0x7fffffffu;
+    const unsigned h = (unsigned)__double2hiint(u);
     return h - 0x39b00000u <= 0x46300000u - 0x39b00000u ? __drcp_rn(u) : __hiloint2double(0x7ff80000, 0);
 }
 
-// a / u with r = rcp_pivot(u), called by all lanes of a warp together.  A numerator outside
-// 2^-700 .. 2^700 (its quotient may leave 2^-800 .. 2^800) is divided plainly, and the whole warp
-// takes that branch, for the warp-collective instructions that follow it.  The check looks at the
-// numerator, not at the quotient, so it is done by the time the quotient is (64 cells, one step:
-// 11.57 ms, 11.70 otherwise).  Zero multipliers are common (a rate that is zero at night) and stay
-// on the short path: a r is then a zero of the right sign, which the correction would lose.
-__device__ __forceinline__ double div_pivot(double a, double u, double r)
+// a / u with r = rcp_pivot(u), called by all lanes of a warp together; bad: r is NaN (or another
+// reason to divide plainly).  A numerator outside 2^-700 .. 2^700 (its quotient may leave
+// 2^-800 .. 2^800) is divided plainly too, and the whole warp takes that branch, for the
+// warp-collective instructions that follow it.  The check looks at the numerator, not at the
+// quotient, so it is done by the time the quotient is (64 cells, one step: 11.57 ms, 11.70
+// otherwise).  Zero multipliers are common (a rate that is zero at night) and stay on the short path:
+// the remainder is taken as u q0 - a, a +0 then, so that the correction is -0 and a zero q0 keeps
+// its sign.
+__device__ __forceinline__ double div_pivot(double a, double u, double r, bool bad)
 {
     const double q0 = a * r;
-    double q = fma(fma(-u, q0, a), r, q0);
-    const bool zero = a == 0.0;
+    double q = fma(-fma(u, q0, -a), r, q0);
     const unsigned h = (unsigned)__double2hiint(a) & 0x7fffffffu;
-    const bool plain = (h - 0x14300000u > 0x6bb00000u - 0x14300000u && !zero) || r != r;
-    if (zero) q = q0;
+    const bool plain = (h - 0x14300000u > 0x6bb00000u - 0x14300000u && a != 0.0) || bad;
     if (__any_sync(0xffffffffu, plain)) {
         const double e = div_exact(a, u);
         if (plain) q = e;
     }
     return q;
 }
+__device__ __forceinline__ double div_pivot(double a, double u, double r) { return div_pivot(a, u, r, r != r); }
 
 // Four quotients of non-negative numbers with one division: the reciprocal of the denominators'
 // product, times the other denominators, is each one's own (simultaneous inversion: P. L.

@@ -40,8 +40,9 @@ constexpr int WIDE_SMEM_BYTES = RADM2_WIDE_SMEM_WORDS * WIDE_BS * 8;
 static __constant__ unsigned char c_wide_rc_rep[RADM2_WIDE_RC_WORDS] = RADM2_WIDE_RC_REP_INIT;
 
 #if RADM2_WIDE_DIV
-#define DIVR(a, u, r) div_pivot(a, u, r)
-#define RCPR(u) rcp_pivot(u)
+// far: a pivot of this attempt has no reciprocal, so all its divisions are plain
+#define DIVR(a, u, r) div_pivot(a, u, r, far)
+#define RCPR(u) [&](double r_) { far = far || r_ != r_; return r_; }(rcp_pivot(u))
 #endif
 
 // Global scratch, word w of the thread (1 KB apart, so every access of a warp is 256 bytes
@@ -189,6 +190,9 @@ __global__ void __launch_bounds__(WIDE_BS, 1) k_rosenbrock_wide(const SolveArgs 
         // LU; a zero pivot is looked for before its row is eliminated (mgpu.cu:2753-2757).  The
         // pivots of rows without eliminations lie side by side and are inverted in a loop.
         bool sing = false;
+#if RADM2_WIDE_DIV
+        bool far = false;
+#endif
 #define LU_PIVOT_CHECK(v) sing = sing | ((v) == 0.0)
 #pragma unroll 4
         for (int k = 0; k < RADM2_WIDE_SPIVOTS; k++) {
