@@ -276,14 +276,30 @@ def per_species_errors(y, ref):
     return out
 
 
-def solver_kernel_name(tuned, args):
-    """The solver kernel the timed arm launched (after autotuning, if any)."""
-    sched, bs, place = args.schedule, args.block_threads, PLACEMENTS[args.placement]
+def launch_shape(tuned, args):
+    """Schedule, threads per block and placement of the timed arm (after autotuning, if any), and
+    whether that is the wide solver (wide_solver in csrc/radm2_capi.cu: asked for, or the library's
+    choice where no shape option is set; the bench sets no rate constants)."""
+    sched, bs, place, bpsm = args.schedule, args.block_threads, PLACEMENTS[args.placement], args.blocks_per_sm
+    minb = cpt = 1
     if tuned is not None:
-        sched, bs = SCHED_NAMES[tuned["chosen"]["schedule"]], tuned["chosen"]["block_threads"]
-        place = tuned["chosen"]["placement"]
+        ch = tuned["chosen"]
+        sched, bs, place, bpsm = SCHED_NAMES[ch["schedule"]], ch["block_threads"], ch["placement"], 0
+        minb, cpt = ch["min_blocks"], ch["cells_per_thread"]
+    asked = place == PLACEMENTS["lu-tmem-wide"] and bs in (0, 128)
+    free = place == PLACEMENTS["global"] and bs == 0 and bpsm <= 0
+    wide = args.precision == "fp64" and sched != "coop" and cpt == 1 and minb <= 1 and (asked or free)
+    return sched, bs, place, wide
+
+
+def solver_kernel_name(tuned, args):
+    """The solver kernel the timed arm launched."""
+    sched, bs, place, wide = launch_shape(tuned, args)
     if sched == "coop":
         return "k_rosenbrock_coop%s_g%d (cooperative solver)" % ("x" if args.parity else "", (bs or 256) // 32)
+    if wide:
+        return "k_rosenbrock_wide<%d> (one cell per thread, cells from a queue%s)" % (
+            1 if args.parity else 0, TMEM_NAMES[PLACEMENTS["lu-tmem-wide"]])
     return "k_rosenbrock (thread-per-cell solver, %s%s)" % (
         sched, TMEM_NAMES.get(place, ""))
 
@@ -593,15 +609,12 @@ def main():
     if os.path.exists(tfile):
         with open(tfile) as f:
             tr = json.load(f)
-        sched_used, place_used = args.schedule, PLACEMENTS[args.placement]
-        if main_arm["tuned"] is not None:
-            sched_used = SCHED_NAMES[main_arm["tuned"]["chosen"]["schedule"]]
-            place_used = main_arm["tuned"]["chosen"]["placement"]
+        sched_used, _, place_used, wide = launch_shape(main_arm["tuned"], args)
         key = "%s-%s" % (args.precision, sched_used)
-        if place_used == PLACEMENTS["lu-tmem"]:
+        if wide:  # cells from a queue in either schedule
+            key = "fp64-persistent-tmemw"
+        elif place_used == PLACEMENTS["lu-tmem"]:
             key += "-tmem"
-        elif place_used == PLACEMENTS["lu-tmem-wide"]:
-            key += "-tmemw"
         if key + "-" + wl in tr:  # a capture of this workload family, if there is one
             key = key + "-" + wl
         if key in tr:
