@@ -1,6 +1,9 @@
 // Divisions of the wide solver: by a number that divides many times over, and four at a time.
 #pragma once
 
+#include <cmath>
+#include <cstring>
+
 namespace radm2 {
 
 static __device__ __noinline__ double div_exact(double a, double u) { return a / u; }
@@ -26,27 +29,42 @@ __device__ __forceinline__ double rcp_pivot(double u)
     return h - 0x39b00000u <= 0x46300000u - 0x39b00000u ? __drcp_rn(u) : __hiloint2double(0x7ff80000, 0);
 }
 
-// a / u with r = rcp_pivot(u), called by all lanes of a warp together; bad: r is NaN (or another
-// reason to divide plainly).  A numerator outside 2^-700 .. 2^700 (its quotient may leave
-// 2^-800 .. 2^800) is divided plainly too, and the whole warp takes that branch, for the
-// warp-collective instructions that follow it.  The check looks at the numerator, not at the
-// quotient, so it is done by the time the quotient is (64 cells, one step: 11.57 ms, 11.70
-// otherwise).  Zero multipliers are common (a rate that is zero at night) and stay on the short path:
-// the remainder is taken as u q0 - a, a +0 then, so that the correction is -0 and a zero q0 keeps
-// its sign.
-__device__ __forceinline__ double div_pivot(double a, double u, double r, bool bad)
+// A double's upper half as a float: magnitudes compare as the doubles' exponents do, sign off by the
+// operand's own modifier (the halves of NaN and of anything beyond 2^1017 compare as too large).
+__device__ __forceinline__ float upper(double a)
+{
+    const int h = __double2hiint(a);
+    float f;
+    memcpy(&f, &h, sizeof f);
+    return f;
+}
+
+constexpr float PIVOT_MAX = 0x1.6p88f, PIVOT_MIN = 0x1.6p-87f;  // uppers of 2^700 and 2^-700
+
+// a / u with r = rcp_pivot(u), called by all lanes of a warp together; limit: PIVOT_MAX, or -1 to
+// divide plainly.  A numerator outside 2^-700 .. 2^700 (its quotient may leave 2^-800 .. 2^800) is
+// divided plainly too, and the whole warp takes that branch, for the warp-collective instructions
+// that follow it.  The check looks at the numerator, not at the quotient, so it is done by the time
+// the quotient is (64 cells, one step: 11.57 ms, 11.70 otherwise), and is three comparisons that
+// pass one predicate on (65,536 cells 50.7 ms, 52.2 with integer operations on the upper half).  Zero multipliers are common (a rate that is zero at night) and stay on the
+// short path: the remainder is taken as u q0 - a, a +0 then, so that the correction is -0 and a zero
+// q0 keeps its sign.
+__device__ __forceinline__ double div_pivot(double a, double u, double r, float limit)
 {
     const double q0 = a * r;
     double q = fma(-fma(u, q0, -a), r, q0);
-    const unsigned h = (unsigned)__double2hiint(a) & 0x7fffffffu;
-    const bool plain = (h - 0x14300000u > 0x6bb00000u - 0x14300000u && a != 0.0) || bad;
+    const float f = fabsf(upper(a));
+    const bool plain = (f < PIVOT_MIN && a != 0.0) || !(f <= limit);
     if (__any_sync(0xffffffffu, plain)) {
         const double e = div_exact(a, u);
         if (plain) q = e;
     }
     return q;
 }
-__device__ __forceinline__ double div_pivot(double a, double u, double r) { return div_pivot(a, u, r, r != r); }
+__device__ __forceinline__ double div_pivot(double a, double u, double r)
+{
+    return div_pivot(a, u, r, r != r ? -1.0f : PIVOT_MAX);
+}
 
 // Four quotients of non-negative numbers with one division: the reciprocal of the denominators'
 // product, times the other denominators, is each one's own (simultaneous inversion: P. L.

@@ -40,9 +40,9 @@ constexpr int WIDE_SMEM_BYTES = RADM2_WIDE_SMEM_WORDS * WIDE_BS * 8;
 static __constant__ unsigned char c_wide_rc_rep[RADM2_WIDE_RC_WORDS] = RADM2_WIDE_RC_REP_INIT;
 
 #if RADM2_WIDE_DIV
-// far: a pivot of this attempt has no reciprocal, so all its divisions are plain
-#define DIVR(a, u, r) div_pivot(a, u, r, far)
-#define RCPR(u) [&](double r_) { far = far || r_ != r_; return r_; }(rcp_pivot(u))
+// limit: -1 once a pivot of this attempt has no reciprocal, so that all its divisions are plain
+#define DIVR(a, u, r) div_pivot(a, u, r, limit)
+#define RCPR(u) [&](double r_) { limit = r_ != r_ ? -1.0f : limit; return r_; }(rcp_pivot(u))
 #endif
 
 // Global scratch, word w of the thread (1 KB apart, so every access of a warp is 256 bytes
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(WIDE_BS, 1) k_rosenbrock_wide(const SolveArgs 
         // pivots of rows without eliminations lie side by side and are inverted in a loop.
         bool sing = false;
 #if RADM2_WIDE_DIV
-        bool far = false;
+        float limit = PIVOT_MAX;
 #endif
 #define LU_PIVOT_CHECK(v) sing = sing | ((v) == 0.0)
 #pragma unroll 4
