@@ -46,9 +46,10 @@ constexpr float PIVOT_MAX = 0x1.6p88f, PIVOT_MIN = 0x1.6p-87f;  // uppers of 2^7
 // divided plainly too, and the whole warp takes that branch, for the warp-collective instructions
 // that follow it.  The check looks at the numerator, not at the quotient, so it is done by the time
 // the quotient is (64 cells, one step: 11.57 ms, 11.70 otherwise), and is three comparisons that
-// pass one predicate on (65,536 cells 50.7 ms, 52.2 with integer operations on the upper half).  Zero multipliers are common (a rate that is zero at night) and stay on the
-// short path: the remainder is taken as u q0 - a, a +0 then, so that the correction is -0 and a zero
-// q0 keeps its sign.
+// pass one predicate on (65,536 cells 50.7 ms, 52.2 with integer operations on the upper half).
+// Zero multipliers are common (a rate that is zero at night) and stay on the short path: the
+// remainder is taken as u q0 - a, a +0 then, so that the correction is -0 and a zero q0 keeps its
+// sign.
 __device__ __forceinline__ double div_pivot(double a, double u, double r, float limit)
 {
     const double q0 = a * r;
